@@ -74,12 +74,6 @@ int guarded(F&& fn) {
 }
 
 
-// host NASA-7 molar enthalpy, same polynomial as the device
-double host_h_molar(const double* c, double T) {
-    const double* a = (T < c[0]) ? c + 1 : c + 8;
-    return kRuniv * T * (a[0] + T * (a[1] * 0.5 + T * (a[2] * (1.0 / 3.0) + T * (a[3] * 0.25 + T * a[4] * 0.2))) + a[5] / T);
-}
-
 void validate_physics(const abl_physics_desc* p) {
     if (!p) throw std::invalid_argument("physics descriptor is NULL");
     if (p->eos != ABL_EOS_PERFECT_GAS && p->eos != ABL_EOS_NASA7) throw std::invalid_argument("unknown eos");
@@ -126,24 +120,40 @@ Phys make_phys(const abl_physics_desc* p) {
     return P;
 }
 
-// upload NASA-7 tables and derived per-species constants; fills P's device pointers
-void upload_species(const abl_physics_desc* p, Phys& P, DevBuf<double>& nasa7, DevBuf<double>& mw, DevBuf<double>& inv_mw, DevBuf<double>& href) {
-    if (p->eos != ABL_EOS_NASA7) return;
+// The rows the device evaluates the NASA-7 species from: per species T_mid, a pad, and for the low and the
+// high range the coefficients of e_k(T) in J/kg (species_poly), then all the 1/W_k. The reference enthalpy
+// is TChemBase's at 298.15 K (tChemBase.cpp:43-69). Extended precision: the formation enthalpy cancels
+// against it to a few per cent of either.
+std::vector<double> thermo_rows(const abl_physics_desc* p) {
     const int ns = p->n_species;
-    std::vector<double> imw(ns), hr(ns);
+    std::vector<double> rows((size_t)(kThermoRow + 1) * ns, 0.0);
     for (int k = 0; k < ns; k++) {
         if (!(p->mw[k] > 0)) throw std::invalid_argument("molar mass must be positive");
-        imw[k] = 1.0 / p->mw[k];
-        hr[k] = host_h_molar(p->nasa7 + 15 * k, kTref) / p->mw[k];  // TChemBase reference enthalpy (tChemBase.cpp:43-69)
+        const double* n7 = p->nasa7 + 15 * (size_t)k;
+        const long double r = (long double)kRuniv / p->mw[k], t = kTref;
+        const double* b = kTref < n7[0] ? n7 + 1 : n7 + 8;
+        const long double href = r * (t * (b[0] + t * (b[1] / 2.0L + t * (b[2] / 3.0L + t * (b[3] / 4.0L + t * b[4] / 5.0L)))) + b[5]);
+        double* row = rows.data() + (size_t)kThermoRow * k;
+        row[0] = n7[0];
+        for (int q = 0; q < 2; q++) {
+            const double* a = n7 + 1 + 7 * q;
+            double* c = row + 2 + 6 * q;
+            c[0] = (double)(r * a[5] - href);
+            c[1] = (double)(r * (a[0] - 1.0L));
+            for (int j = 1; j < 5; j++) c[1 + j] = (double)(r * a[j] / (j + 1.0L));
+        }
+        rows[(size_t)kThermoRow * ns + k] = 1.0 / p->mw[k];
     }
-    nasa7.upload(p->nasa7, (size_t)ns * 15);
-    mw.upload(p->mw, ns);
-    inv_mw.upload(imw.data(), ns);
-    href.upload(hr.data(), ns);
-    P.nasa7 = nasa7.p;
-    P.mw = mw.p;
-    P.inv_mw = inv_mw.p;
-    P.href = href.p;
+    return rows;
+}
+
+// upload the species' rows; fills P's device pointers
+void upload_species(const abl_physics_desc* p, Phys& P, DevBuf<double>& thermo) {
+    if (p->eos != ABL_EOS_NASA7) return;
+    const std::vector<double> rows = thermo_rows(p);
+    thermo.upload(rows.data(), rows.size());
+    P.thermo = thermo.p;
+    P.inv_mw = thermo.p + (size_t)kThermoRow * p->n_species;
 }
 
 // ---- dispatch over the compiled (DIM, NS) instances ------------------------------------------------
@@ -362,26 +372,30 @@ __device__ void eos_property(const Phys& P, int ns, int prop, const double* U, b
     double ys[kMaxSpecies];
     fill_y(ns, rho, U + 2 + DIM, ys);
     switch (prop) {
-        case ABL_PROP_PRESSURE: *out = rho * kRuniv * T / mixture_mw(P, ns, ys); return;
+        case ABL_PROP_PRESSURE: *out = rho * kRuniv * T * mixture_imw(P, ns, ys); return;
         case ABL_PROP_TEMPERATURE: *out = temperature<DIM, kMaxSpecies>(P, ns, U, T, ok); return;
-        case ABL_PROP_INTERNAL_SENSIBLE_ENERGY: *out = e_sens(P, ns, ys, T); return;
+        case ABL_PROP_INTERNAL_SENSIBLE_ENERGY: {
+            MixPoly m;
+            mix_poly(P, ns, ys, T, &m);
+            *out = poly_e(m.c, T);
+            return;
+        }
         case ABL_PROP_SENSIBLE_ENTHALPY: {
             double h = 0;
-            for (int k = 0; k < ns; k++) h += (nasa_h_molar(P.nasa7 + 15 * k, T) * P.inv_mw[k] - P.href[k]) * ys[k];
+            for (int k = 0; k < ns; k++) h += species_h(P, k, T) * ys[k];
             *out = h;
             return;
         }
-        case ABL_PROP_CV: *out = mixture_cp(P, ns, ys, T) - kRuniv / mixture_mw(P, ns, ys); return;
-        case ABL_PROP_CP: *out = mixture_cp(P, ns, ys, T); return;
+        case ABL_PROP_CV: *out = mixture_cv(P, ns, ys, T); return;
+        case ABL_PROP_CP: *out = mixture_cv(P, ns, ys, T) + kRuniv * mixture_imw(P, ns, ys); return;
         case ABL_PROP_SPEED_OF_SOUND: {
-            const double cp = mixture_cp(P, ns, ys, T);
-            const double R = kRuniv / mixture_mw(P, ns, ys);
-            const double cv = cp - R;
-            *out = sqrt(cp / cv * R * T);
+            const double cv = mixture_cv(P, ns, ys, T);
+            const double R = kRuniv * mixture_imw(P, ns, ys);
+            *out = sqrt((cv + R) / cv * R * T);
             return;
         }
         case ABL_PROP_SPECIES_SENSIBLE_ENTHALPY:
-            for (int k = 0; k < ns; k++) out[k] = nasa_h_molar(P.nasa7 + 15 * k, T) * P.inv_mw[k] - P.href[k];
+            for (int k = 0; k < ns; k++) out[k] = species_h(P, k, T);
             return;
         case ABL_PROP_DENSITY: *out = rho; return;
     }
@@ -410,9 +424,9 @@ int status_to_code(int bits) {
 }  // namespace
 
 // ---- allocation-free EOS batch ----------------------------------------------------------------------
-// Scratch of abl_eos_batch_noalloc: the NASA-7 tables the kernel reads (T_mid + 14 coefficients, molar
-// mass, 1/molar mass, reference enthalpy per species) followed by the status word. 16 KiB, held by every
-// GPU that loads this library until the process exits; 64 species need 9,216 bytes.
+// Scratch of abl_eos_batch_noalloc: the species' rows that the kernel reads (thermo_rows) followed by the
+// status word. 16 KiB, held by every GPU that loads this library until the process exits; 64 species need
+// 7,680 bytes.
 constexpr int kNoAllocMaxSpecies = 64;
 constexpr size_t kNoAllocScratchBytes = 16384;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
@@ -530,7 +544,7 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
         fv->need_aux_grad = dif;
         // the mixture EOS keeps T resident (secant guess + face temperatures); a perfect gas recomputes it
         fv->need_aux = physics->eos == ABL_EOS_NASA7;
-        upload_species(physics, fv->phys, fv->nasa7, fv->mw, fv->inv_mw, fv->href);
+        upload_species(physics, fv->phys, fv->thermo);
         if (physics->species_diff && physics->species_diffusion) {
             fv->diff_k.upload(physics->species_diff, physics->n_species);
             fv->phys.diff_k = fv->diff_k.p;
@@ -1225,8 +1239,8 @@ int abl_eos_batch(const abl_physics_desc* physics, int dim, int property, int64_
         if (n < 0 || (n > 0 && (!conserved || !out))) throw std::invalid_argument("NULL argument");
         if (n == 0) return;
         Phys P = make_phys(physics);
-        DevBuf<double> nasa7, mw, inv_mw, href;
-        upload_species(physics, P, nasa7, mw, inv_mw, href);
+        DevBuf<double> thermo;
+        upload_species(physics, P, thermo);
         const int ns = physics->n_species;
         const int nc = 2 + dim + ns;
         const int psz = property == ABL_PROP_SPECIES_SENSIBLE_ENTHALPY ? ns : 1;
@@ -1267,32 +1281,17 @@ int abl_eos_batch_noalloc(const abl_physics_desc* physics, int dim, int property
         unsigned char* scratch = noalloc_scratch();
         if (n == 0) return;
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        // layout: nasa7 [ns][15] | mw [ns] | 1/mw [ns] | h_ref [ns] | status (int)
-        double* d_nasa7 = reinterpret_cast<double*>(scratch);
-        double* d_mw = d_nasa7 + 15 * kNoAllocMaxSpecies;
-        double* d_imw = d_mw + kNoAllocMaxSpecies;
-        double* d_href = d_imw + kNoAllocMaxSpecies;
-        int* d_status = reinterpret_cast<int*>(d_href + kNoAllocMaxSpecies);
-        static_assert((15 + 3) * kNoAllocMaxSpecies * sizeof(double) + sizeof(int) <= kNoAllocScratchBytes, "scratch too small");
+        // layout: thermo rows [ns][14] | 1/mw [ns], then the status word
+        double* d_rows = reinterpret_cast<double*>(scratch);
+        int* d_status = reinterpret_cast<int*>(d_rows + (kThermoRow + 1) * kNoAllocMaxSpecies);
+        static_assert((kThermoRow + 1) * kNoAllocMaxSpecies * sizeof(double) + sizeof(int) <= kNoAllocScratchBytes, "scratch too small");
         Phys P = make_phys(physics);
         if (physics->eos == ABL_EOS_NASA7) {
-            std::vector<double> tables(18 * (size_t)ns);
-            for (int k = 0; k < ns; k++) {
-                if (!(physics->mw[k] > 0)) throw std::invalid_argument("molar mass must be positive");
-                tables[15 * (size_t)ns + k] = physics->mw[k];
-                tables[16 * (size_t)ns + k] = 1.0 / physics->mw[k];
-                tables[17 * (size_t)ns + k] = host_h_molar(physics->nasa7 + 15 * k, kTref) / physics->mw[k];
-            }
-            std::memcpy(tables.data(), physics->nasa7, 15 * (size_t)ns * sizeof(double));
-            // pageable host source: the copy is staged before cudaMemcpyAsync returns, so `tables` may go
-            ABL_CUDA(cudaMemcpyAsync(d_nasa7, tables.data(), 15 * (size_t)ns * sizeof(double), cudaMemcpyHostToDevice, s));
-            ABL_CUDA(cudaMemcpyAsync(d_mw, tables.data() + 15 * (size_t)ns, (size_t)ns * sizeof(double), cudaMemcpyHostToDevice, s));
-            ABL_CUDA(cudaMemcpyAsync(d_imw, tables.data() + 16 * (size_t)ns, (size_t)ns * sizeof(double), cudaMemcpyHostToDevice, s));
-            ABL_CUDA(cudaMemcpyAsync(d_href, tables.data() + 17 * (size_t)ns, (size_t)ns * sizeof(double), cudaMemcpyHostToDevice, s));
-            P.nasa7 = d_nasa7;
-            P.mw = d_mw;
-            P.inv_mw = d_imw;
-            P.href = d_href;
+            const std::vector<double> rows = thermo_rows(physics);
+            // pageable host source: the copy is staged before cudaMemcpyAsync returns, so `rows` may go
+            ABL_CUDA(cudaMemcpyAsync(d_rows, rows.data(), rows.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+            P.thermo = d_rows;
+            P.inv_mw = d_rows + (size_t)kThermoRow * ns;
         }
         // the status word is the one scratch entry read before it is written: clear it every call
         ABL_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), s));

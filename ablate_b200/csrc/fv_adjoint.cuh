@@ -48,12 +48,6 @@ ABL_HD void internal_energy_vjp(const double* U, double eb, double* Ub) {
     Ub[0] -= eb * (U[1] - vu) * irho * irho;
 }
 
-template <class S>
-ABL_HD S nasa_dcp_molar(const double* c, S T) {
-    const double* a = (T < c[0]) ? c + 1 : c + 8;
-    return kRuniv * (a[1] + T * (2.0 * a[2] + T * (3.0 * a[3] + T * 4.0 * a[4])));
-}
-
 // reverse of fill_y (clip to [0, 1], renormalise or close with the last species)
 template <int NSMAX>
 ABL_HD void fill_y_vjp(int ns, double rho, const double* rhoY, const double* ysb, double* rhob, double* rhoYb) {
@@ -86,13 +80,17 @@ ABL_UNROLL_SPECIES
 // reverse of the mixture temperature T(e_ref, Y) (implicit function of e_s(T, Y) = e_ref)
 template <int DIM, int NSMAX>
 ABL_HD void nasa_temperature_vjp(const Phys& P, int ns, const double* U, const double* ys, double T, double Tb, double* ysb, double* Ub) {
-    double cv = 0;
+    double cv = 0, ek[NSMAX > 0 ? NSMAX : 1];
 ABL_UNROLL_SPECIES
-    for (int k = 0; k < ns; k++) cv += ys[k] * (nasa_cp_molar(P.nasa7 + 15 * k, T) - kRuniv) * P.inv_mw[k];
+    for (int k = 0; k < ns; k++) {
+        double c[6];
+        species_poly(P, k, T, c);
+        cv += ys[k] * poly_cv(c, T);
+        ek[k] = poly_e(c, T);
+    }
     const double q = Tb / cv;
 ABL_UNROLL_SPECIES
-    for (int k = 0; k < ns; k++)
-        ysb[k] -= q * (nasa_h_molar(P.nasa7 + 15 * k, T) * P.inv_mw[k] - P.href[k] - kRuniv * T * P.inv_mw[k]);
+    for (int k = 0; k < ns; k++) ysb[k] -= q * ek[k];
     internal_energy_vjp<DIM>(U, q, Ub);
 }
 
@@ -112,33 +110,32 @@ ABL_HD void decode_vjp(const Phys& P, int ns, const double* U, const Decoded<dou
     double ys[NY], ysb[NY];
     fill_y(ns, rho, U + 2 + DIM, ys);
     const double T = dd.T;
-    double cp = 0, iw = 0, dcp = 0;
+    // one pass over the species at T: e_k and c_v,k serve the energy, the sound speed and the temperature's
+    // own reverse (e_s(T, Y) = e_ref)
+    double cv = 0, iw = 0, dcv = 0, ek[NY], ck[NY];
 ABL_UNROLL_SPECIES
     for (int k = 0; k < ns; k++) {
-        cp += ys[k] * nasa_cp_molar(P.nasa7 + 15 * k, T) * P.inv_mw[k];
-        dcp += ys[k] * nasa_dcp_molar(P.nasa7 + 15 * k, T) * P.inv_mw[k];
+        double c[6];
+        species_poly(P, k, T, c);
+        ek[k] = poly_e(c, T);
+        ck[k] = poly_cv(c, T);
+        cv += ys[k] * ck[k];
+        dcv += ys[k] * poly_dcv(c, T);
         iw += ys[k] * P.inv_mw[k];
-        ysb[k] = 0.0;
     }
-    const double R = kRuniv * rcp64(rcp64(iw));
-    const double cv = cp - R;
-    const double gamma = cp * rcp64(cv);
-    const double q = dd.a > 0 ? ab / (2.0 * dd.a) : 0.0;  // a = sqrt(gamma R T)
+    const double R = kRuniv * iw, icv = rcp64(cv);
+    const double gamma = (cv + R) * icv;
+    const double q = dd.a > 0 ? ab / (2.0 * dd.a) : 0.0;  // a = sqrt(gamma R T), gamma = 1 + R / cv
     const double gb = q * R * T;
-    double Rb = q * gamma * T + pb * rho * T;
-    double Tb = q * gamma * R + pb * rho * R;
+    const double cvb = -gb * R * icv * icv;
+    const double Rb = q * gamma * T + pb * rho * T + gb * icv;
+    // e = e_s(T, Y): de/dT = cv, de/dY_k = e_k
+    const double Tb = q * gamma * R + pb * rho * R + cvb * dcv + eb * cv;
     Ub[0] += pb * R * T;
-    const double cpb = -gb * R / (cv * cv);
-    Rb += gb * cp / (cv * cv);
-    Tb += cpb * dcp;
-    // e = e_s(T, Y): de/dT = cv, de/dY_k = e_s,k
+    const double qT = Tb * icv;
 ABL_UNROLL_SPECIES
-    for (int k = 0; k < ns; k++) {
-        const double esk = nasa_h_molar(P.nasa7 + 15 * k, T) * P.inv_mw[k] - P.href[k] - kRuniv * T * P.inv_mw[k];
-        ysb[k] += eb * esk + cpb * nasa_cp_molar(P.nasa7 + 15 * k, T) * P.inv_mw[k] + Rb * kRuniv * P.inv_mw[k];
-    }
-    Tb += eb * cv;
-    nasa_temperature_vjp<DIM, NSMAX>(P, ns, U, ys, T, Tb, ysb, Ub);
+    for (int k = 0; k < ns; k++) ysb[k] = (eb - qT) * ek[k] + cvb * ck[k] + Rb * kRuniv * P.inv_mw[k];
+    internal_energy_vjp<DIM>(U, qT, Ub);
     fill_y_vjp<NSMAX>(ns, rho, U + 2 + DIM, ysb, Ub, Ub + 2 + DIM);
 }
 
@@ -149,13 +146,15 @@ ABL_HD void cp_at_vjp(const Phys& P, int ns, const double* U, double T, double c
     constexpr int NY = NSMAX > 0 ? NSMAX : 1;
     double ys[NY], ysb[NY];
     fill_y(ns, U[0], U + 2 + DIM, ys);
-    double dcp = 0;
+    double dcv = 0;
 ABL_UNROLL_SPECIES
     for (int k = 0; k < ns; k++) {
-        dcp += ys[k] * nasa_dcp_molar(P.nasa7 + 15 * k, T) * P.inv_mw[k];
-        ysb[k] = cpb * nasa_cp_molar(P.nasa7 + 15 * k, T) * P.inv_mw[k];
+        double c[6];
+        species_poly(P, k, T, c);
+        dcv += ys[k] * poly_dcv(c, T);
+        ysb[k] = cpb * (poly_cv(c, T) + kRuniv * P.inv_mw[k]);
     }
-    *Tb += cpb * dcp;
+    *Tb += cpb * dcv;
     fill_y_vjp<NSMAX>(ns, U[0], U + 2 + DIM, ysb, Ub, Ub + 2 + DIM);
 }
 
@@ -619,7 +618,14 @@ ABL_UNROLL_SPECIES
             double rhob = 0, Tb = 0;
 ABL_UNROLL_SPECIES
             for (int s = 0; s < NS; ++s) {
-                const double hs = P.eos == ABL_EOS_NASA7 ? nasa_h_molar(P.nasa7 + 15 * s, fa[0]) * P.inv_mw[s] - P.href[s] : 0.0;
+                double hs = 0.0, cps = 0.0;
+                if (P.eos == ABL_EOS_NASA7) {
+                    double c[6];
+                    species_poly(P, s, fa[0], c);
+                    const double r = kRuniv * P.inv_mw[s];
+                    hs = poly_e(c, fa[0]) + r * fa[0];
+                    cps = poly_cv(c, fa[0]) + r;
+                }
                 // one constant D_k per species (no state dependence), or the transport model's D
                 const double Ds = P.diff_k ? P.diff_k[s] : diff;
                 double hsb = 0;
@@ -632,7 +638,7 @@ ABL_UNROLL_SPECIES
                     gfb[yoff + s * DIM + d] += q * density * Ds;
                     hsb -= normal[d] * density * Ds * gy * fb[1];
                 }
-                if (P.eos == ABL_EOS_NASA7) Tb += hsb * nasa_cp_molar(P.nasa7 + 15 * s, fa[0]) * P.inv_mw[s];
+                Tb += hsb * cps;
             }
             fsb[0] += rhob;
             fab[0] += Tb;

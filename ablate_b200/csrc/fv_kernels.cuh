@@ -534,13 +534,11 @@ __device__ __forceinline__ void advection_split(const Phys& P, const double* nor
         } else {
             double ys[NS > 0 ? NS : 1];
             fill_y(NS, rho, u + 2 + DIM, ys);
-            const double T = nasa_temperature(P, NS, ys, eint, guess[s], ok);
-            e[s] = e_sens(P, NS, ys, T);
-            const double cp = mixture_cp(P, NS, ys, T);
-            const double mw = mixture_mw(P, NS, ys);
-            const double R = kRuniv / mw;
-            p[s] = rho * kRuniv * T / mw;
-            a[s] = sqrtf(float(cp / (cp - R) * R * T));
+            double cv;
+            const double T = nasa_temperature_s<NS>(P, NS, ys, eint, guess[s], ok, &cv, &e[s]);
+            const double R = kRuniv * mixture_imw(P, NS, ys);
+            p[s] = rho * R * T;
+            a[s] = sqrtf(float((cv + R) / cv * R * T));
         }
     }
     SplitFlux sf = (P.flux == ABL_FLUX_AUSM) ? flux_split<ABL_FLUX_AUSM>(P, uL[0], p[0], unA[0], a[0], uR[0], p[1], unA[1], a[1], area)
@@ -775,7 +773,7 @@ ABL_UNROLL_SPECIES
                 S hs[NS];
                 if (P.eos == ABL_EOS_NASA7) {
 ABL_UNROLL_SPECIES
-                    for (int s = 0; s < NS; s++) hs[s] = nasa_h_molar(P.nasa7 + 15 * s, fa[0]) * P.inv_mw[s] - P.href[s];
+                    for (int s = 0; s < NS; s++) hs[s] = species_h(P, s, fa[0]);
                 } else {
 ABL_UNROLL_SPECIES
                     for (int s = 0; s < NS; s++) hs[s] = 0.0;
