@@ -579,20 +579,24 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
             return b.tf_cells.size() < a.tf_cells.size() ? b : a;
         };
         // and whose shared memory fits every pass: the face fluxes (value and tangent pairs in the JVP) and
-        // the adjoint's per-cell accumulator rows (state, gradient, aux, aux gradient; odd stride)
+        // the adjoint's face records (AdjRow::R)
         const int naux_ = 1 + h.dim + physics->n_species;
-        const size_t adj_row = (size_t)((nc_ + nc_ * h.dim + naux_ + naux_ * h.dim) | 1) * sizeof(double);
-        auto fits = [&](const Tiles& t, int cells) {
+        const size_t adj_row = (size_t)std::max(naux_ + 2 + h.dim + physics->n_species, 2 * nc_) * sizeof(double);
+        auto fits = [&](const Tiles& t) {
             const size_t faces = (size_t)std::max(t.max_faces, 1) * nc_ * sizeof(double);
-            return faces <= 200 * 1024 && 2 * faces <= 227 * 1024 && (size_t)cells * adj_row <= 227 * 1024;
+            return faces <= 200 * 1024 && 2 * faces <= 227 * 1024 && (size_t)std::max(t.max_faces, 1) * adj_row <= 227 * 1024;
         };
-        int tile = 256;
+        // 256 cells, or 128 with species: a tile's face records of either pass then leave room for the CTAs
+        // that the registers allow (five species, 256 cells: one CTA of the adjoint per SM instead of three)
+        int tile = physics->n_species > 0 && !fused_enabled() ? 128 : 256;
         Tiles tl = tiles_for(tile);
-        while (!fits(tl, tile) && tile > 16) {
+        while (!fits(tl) && tile > 16) {
             tile /= 2;
             tl = tiles_for(tile);
         }
-        fv->tile_smem = (int)((size_t)std::max(tl.max_faces, 1) * nc_ * sizeof(double));
+        fv->tile_max_faces = std::max(tl.max_faces, 1);
+        fv->tile_cells_max = tile;
+        fv->tile_smem = (int)((size_t)fv->tile_max_faces * nc_ * sizeof(double));
         std::vector<uint16_t> geo_cls;  // per tile face record its geometry record (kept for the fused tables)
         fv->tile_cell_ptr.upload(tl.cell_ptr.data(), tl.cell_ptr.size());
         fv->tile_cells.upload(tl.cells.data(), tl.cells.size());
@@ -624,14 +628,9 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
         }
         fv->tc_fptr.upload(tl.tc_fptr.data(), tl.tc_fptr.size());
         fv->tc_face.upload(tl.tc_face.data(), tl.tc_face.size());
-        fv->col_base.upload(tl.col_base.data(), tl.col_base.size());
-        fv->col_start.upload(tl.col_start.data(), tl.col_start.size());
-        fv->tf_slot.upload(tl.tf_slot.data(), tl.tf_slot.size());
-        fv->tf_adj.upload(tl.tf_adj.data(), tl.tf_adj.size());
         fv->tf_nb.upload(tl.tf_nb.data(), tl.tf_nb.size());
         fv->face_nb.upload(tl.face_nb.data(), tl.face_nb.size());
         fv->n_nb = tl.n_nb;
-        for (int k = 0; k < tl.n_tiles; k++) fv->tile_max_cells = std::max(fv->tile_max_cells, tl.cell_ptr[k + 1] - tl.cell_ptr[k]);
         {
             std::vector<int32_t> no, ow;
             for (int c = 0; c < h.n_cells; c++) (h.kind[c] != ABL_CELL_OWNED ? no : ow).push_back(c);
@@ -822,10 +821,6 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
         M.tf_geo = fv->tf_geo.p;
         M.tc_fptr = fv->tc_fptr.p;
         M.tc_face = fv->tc_face.p;
-        M.tf_adj = fv->tf_adj.p;
-        M.col_base = fv->col_base.p;
-        M.col_start = fv->col_start.p;
-        M.tf_slot = fv->tf_slot.p;
         M.tf_nb = fv->tf_nb.p;
         M.face_nb = fv->face_nb.p;
         M.n_nonowned = (int)fv->nonowned.n;

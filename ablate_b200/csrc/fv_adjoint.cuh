@@ -9,12 +9,11 @@
 // keeps anyway, plus the unlimited gradient, the limiter factor and the minimising face per component.
 // Every per-face intermediate (face states, EOS decode, flux calculator) is recomputed:
 //   k_gradient          forward gradients, with the limiter records
-//   k_tile_adjoint      one CTA per tile. Per face, colour by colour: recompute the face states, the
-//                       EOS decode and the flux calculator, then run the flux backwards; the adjoint of
-//                       each side's state, limited gradient, aux and aux gradient is summed into that
-//                       cell's shared-memory accumulators (faces of one colour touch distinct cells, so
-//                       no atomics and a fixed order). Then per tile cell the limiter and least-squares
-//                       gradient are run backwards from the records of the forward gradient pass.
+//   k_tile_adjoint      one CTA per tile. Per face: recompute the face states, the EOS decode and the flux
+//                       calculator, then run the flux backwards into the face's shared-memory record.
+//                       Per tile cell: sum the adjoints of its state, limited gradient, aux and aux
+//                       gradient from its faces' records, then run the limiter and the least-squares
+//                       gradient backwards from the records of the forward gradient pass.
 //   k_adjoint_nonowned  the same cell step for boundary ghosts and halos, from per-face records.
 //   k_adjoint_gather    per cell: the neighbour terms of the gradient, limiter and aux-gradient adjoints
 //                       (a gather over the cell's faces, the transpose of the forward gathers), then the
@@ -436,17 +435,27 @@ ABL_HD void calc_vjp(const Phys& P, const double* x, double mfb, double p12b, do
 // ---------------------------------------------------------------------------------------------------
 // face fluxes backwards
 // ---------------------------------------------------------------------------------------------------
-// Two lanes per face: lanes 2j (left side) and 2j+1 (right side) of a warp hold one face. Each lane
-// projects, decodes and reverses its own side; what couples the sides (the flux calculator and the
-// upwind choice, the averaged face state of the diffusion flux) is exchanged with the partner lane and
-// evaluated identically in both. Every exchange sits in control flow both lanes take.
-__device__ __forceinline__ double xch(unsigned mask, double v) { return __shfl_xor_sync(mask, v, 1); }
+// One side of the advection flux backwards: eb, pb, irhob, velb and ub arrive with the upwind terms; the
+// flux calculator's adjoints of (u.n, a, rho, p) on this side are g[0..3]. ub is this side's face state.
+template <int DIM, int NS>
+__device__ __forceinline__ void advection_side_vjp(const Phys& P, const double* norm, const double* u, double irho, const Decoded<double>& dd,
+                                                   const double* g, double eb, double pb, double irhob, double* velb, double* ub) {
+    ub[0] += g[2];
+#pragma unroll
+    for (int d = 0; d < DIM; d++) {
+        velb[d] += g[0] * norm[d];
+        ub[2 + d] += velb[d] * irho;
+        irhob += velb[d] * u[2 + d];
+    }
+    ub[0] -= irhob * irho * irho;
+    decode_vjp<DIM, NS>(P, NS, u, dd, eb, g[1], pb + g[3], ub);
+}
 
-// advection (NavierStokesTransport::AdvectionFlux + SpeciesTransport::AdvectionFlux) backwards for
-// this lane's side: fb = flux adjoint, ub += adjoint of this side's projected face state u
+// advection (NavierStokesTransport::AdvectionFlux + SpeciesTransport::AdvectionFlux) backwards: fb = flux
+// adjoint, ubL and ubR = adjoints of the two projected face states
 template <int DIM, int NS, int FK>
-__device__ __forceinline__ void advection_vjp_side(const Phys& P, unsigned mask, int side, const double* normal, const double* u, double Tguess,
-                                                   bool adv, bool spadv, const double* fb, double* ub, bool* ok, bool* rok) {
+__device__ __forceinline__ void advection_vjp(const Phys& P, const double* normal, const double* uL, const double* uR, double gsL, double gsR,
+                                              bool adv, bool spadv, const double* fb, double* ubL, double* ubR, bool* ok, bool* rok) {
     using D = Dims<DIM, NS>;
     double areaMag = 0;
 #pragma unroll
@@ -456,114 +465,108 @@ __device__ __forceinline__ void advection_vjp_side(const Phys& P, unsigned mask,
     double norm[DIM];
 #pragma unroll
     for (int d = 0; d < DIM; d++) norm[d] = normal[d] * iA;
-    const auto dd = decode<DIM, NS>(P, NS, u, Tguess, ok);
-    const double rho = u[0], irho = rcp64(rho);
-    double vel[DIM], un = 0, v2 = 0;
+    const auto dL = decode<DIM, NS>(P, NS, uL, gsL, ok);
+    const auto dR = decode<DIM, NS>(P, NS, uR, gsR, ok);
+    const double irL = rcp64(uL[0]), irR = rcp64(uR[0]);
+    double velL[DIM], velR[DIM], unL = 0, unR = 0;
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
-        vel[d] = u[2 + d] * irho;
-        un += vel[d] * norm[d];
-        v2 += vel[d] * vel[d];
+        velL[d] = uL[2 + d] * irL;
+        unL += velL[d] * norm[d];
+        velR[d] = uR[2 + d] * irR;
+        unR += velR[d] * norm[d];
     }
-    const double vm = sqrt(v2);
-    const double H = dd.e + vm * vm / 2.0 + dd.p * irho;
-    // the flux calculator on both sides' values, in (left, right) order in both lanes
-    const double un_o = xch(mask, un), a_o = xch(mask, dd.a), rho_o = xch(mask, rho), p_o = xch(mask, dd.p);
-    const double x[8] = {side ? un_o : un, side ? a_o : dd.a, side ? rho_o : rho, side ? p_o : dd.p,
-                         side ? un : un_o, side ? dd.a : a_o, side ? rho : rho_o, side ? dd.p : p_o};
+    const double x[8] = {unL, dL.a, uL[0], dL.p, unR, dR.a, uR[0], dR.p};
     double mf, p12;
     const int dir = flux_calc_k<FK, double>(P, x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7], &mf, &p12, rok);
     const double mA = mf * areaMag;
-    const double H_o = xch(mask, H);
-    double vel_o[DIM];
+    // LEFT upwinds side L, RIGHT side R, no direction half of each; for the species anything but LEFT is R
+    const double wL = dir == ABL_DIR_LEFT ? 1.0 : (dir == ABL_DIR_RIGHT ? 0.0 : 0.5), wR = 1.0 - wL;
+    double mfb = 0, p12b = 0, ebL = 0, ebR = 0, pbL = 0, pbR = 0, ibL = 0, ibR = 0, vbL[DIM], vbR[DIM];
 #pragma unroll
-    for (int d = 0; d < DIM; d++) vel_o[d] = xch(mask, vel[d]);
-    // LEFT upwinds side 0, RIGHT side 1; for the species anything but LEFT takes side 1
-    const bool upme = (dir == ABL_DIR_LEFT) == (side == 0);
-    double mfb = 0, p12b = 0, eb = 0, pb = 0, irhob = 0, velb[DIM];
-#pragma unroll
-    for (int d = 0; d < DIM; d++) velb[d] = 0.0;
+    for (int d = 0; d < DIM; d++) vbL[d] = vbR[d] = 0.0;
+ABL_UNROLL_SPECIES
+    for (int k = 0; k < D::NC; k++) ubL[k] = ubR[k] = 0.0;
     if (adv) {
-        mfb += areaMag * fb[0];
+        double v2L = 0, v2R = 0;
 #pragma unroll
-        for (int n = 0; n < DIM; n++) p12b += normal[n] * fb[2 + n];
-        if (dir == ABL_DIR_LEFT || dir == ABL_DIR_RIGHT) {
-            double sacc = (upme ? H : H_o) * fb[1];
+        for (int d = 0; d < DIM; d++) {
+            v2L += velL[d] * velL[d];
+            v2R += velR[d] * velR[d];
+        }
+        const double HL = dL.e + 0.5 * v2L + dL.p * irL, HR = dR.e + 0.5 * v2R + dR.p * irR;
+        mfb = areaMag * fb[0];
+        double sacc = (wL * HL + wR * HR) * fb[1];
 #pragma unroll
-            for (int n = 0; n < DIM; n++) sacc += (upme ? vel[n] : vel_o[n]) * fb[2 + n];
-            mfb += areaMag * sacc;
-            if (upme) {
-                const double Hb = mA * fb[1];
-                eb += Hb;
-                pb += Hb * irho;
-                irhob += Hb * dd.p;
+        for (int n = 0; n < DIM; n++) {
+            p12b += normal[n] * fb[2 + n];
+            sacc += (wL * velL[n] + wR * velR[n]) * fb[2 + n];
+        }
+        mfb += areaMag * sacc;
+        const double Hb = mA * fb[1];
+        ebL = wL * Hb;
+        ebR = wR * Hb;
+        pbL = ebL * irL;
+        pbR = ebR * irR;
+        ibL = ebL * dL.p;
+        ibR = ebR * dR.p;
 #pragma unroll
-                for (int n = 0; n < DIM; n++) velb[n] += Hb * vel[n] + mA * fb[2 + n];
-            }
-        } else {
-            double sacc = 0.5 * (H + H_o) * fb[1];
-#pragma unroll
-            for (int n = 0; n < DIM; n++) sacc += 0.5 * (vel[n] + vel_o[n]) * fb[2 + n];
-            mfb += areaMag * sacc;
-            const double Hb = 0.5 * mA * fb[1];
-            eb += Hb;
-            pb += Hb * irho;
-            irhob += Hb * dd.p;
-#pragma unroll
-            for (int n = 0; n < DIM; n++) velb[n] += Hb * vel[n] + 0.5 * mA * fb[2 + n];
+        for (int n = 0; n < DIM; n++) {
+            vbL[n] = ebL * velL[n] + wL * mA * fb[2 + n];
+            vbR[n] = ebR * velR[n] + wR * mA * fb[2 + n];
         }
     }
     if (NS > 0 && spadv && dir == ABL_DIR_NA && P.sp_compact) {
         // compact process, no direction: flux_s = mA (rhoY_L + rhoY_R) / (rho_L + rho_R) (both halves)
-        const double rhoM = 0.5 * (rho + rho_o), irm = 1.0 / rhoM;
+        const double irm = 1.0 / (0.5 * (uL[0] + uR[0]));
 ABL_UNROLL_SPECIES
         for (int s = 0; s < NS; s++) {
-            const double ry = u[D::NE + s], ry_o = xch(mask, ry);
-            const double num = 0.5 * (side ? ry + ry_o : ry_o + ry);
+            const double num = 0.5 * (uL[D::NE + s] + uR[D::NE + s]);
             mfb += areaMag * num * irm * fb[D::NE + s];
-            ub[D::NE + s] += 0.5 * mA * irm * fb[D::NE + s];
-            ub[0] -= 0.5 * mA * num * irm * irm * fb[D::NE + s];
+            const double yb = 0.5 * mA * irm * fb[D::NE + s], rb = yb * num * irm;
+            ubL[D::NE + s] = yb;
+            ubR[D::NE + s] = yb;
+            ubL[0] -= rb;
+            ubR[0] -= rb;
         }
     } else if (NS > 0 && spadv) {
+        const bool left = dir == ABL_DIR_LEFT;
+        const double ir = left ? irL : irR;
+        double ib = 0;
 ABL_UNROLL_SPECIES
         for (int s = 0; s < NS; s++) {
-            const double Y = u[D::NE + s] * irho;
-            const double Y_o = xch(mask, Y);
-            mfb += areaMag * (upme ? Y : Y_o) * fb[D::NE + s];
-            if (upme) {
-                const double Yb = mA * fb[D::NE + s];
-                ub[D::NE + s] += Yb * irho;
-                irhob += Yb * u[D::NE + s];
-            }
+            const double ry = left ? uL[D::NE + s] : uR[D::NE + s], Yb = mA * fb[D::NE + s];
+            mfb += areaMag * (ry * ir) * fb[D::NE + s];
+            ubL[D::NE + s] = left ? Yb * ir : 0.0;
+            ubR[D::NE + s] = left ? 0.0 : Yb * ir;
+            ib += Yb * ry;
         }
+        if (left)
+            ibL += ib;
+        else
+            ibR += ib;
     }
     double g[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (mfb != 0.0 || p12b != 0.0) calc_vjp<FK>(P, x, mfb, p12b, g, rok);
-    const double gu = side ? g[4] : g[0], ga = side ? g[5] : g[1], gr = side ? g[6] : g[2], gp = side ? g[7] : g[3];
-    ub[0] += gr;
-#pragma unroll
-    for (int d = 0; d < DIM; d++) {
-        velb[d] += gu * norm[d];
-        ub[2 + d] += velb[d] * irho;
-        irhob += velb[d] * u[2 + d];
-    }
-    ub[0] -= irhob * irho * irho;
-    decode_vjp<DIM, NS>(P, NS, u, dd, eb, ga, pb + gp, ub);
+    advection_side_vjp<DIM, NS>(P, norm, uL, irL, dL, g, ebL, pbL, ibL, vbL, ubL);
+    advection_side_vjp<DIM, NS>(P, norm, uR, irR, dR, g + 4, ebR, pbR, ibR, vbR, ubR);
 }
 
-// diffusion (NavierStokesTransport::DiffusionFlux, SpeciesTransport diffusion) backwards. fs, fa and
-// gf are the face state, aux and aux gradient (averages of the two cells); each side receives half of
-// the returned fsb, fab, gfb.
+// diffusion (NavierStokesTransport::DiffusionFlux, SpeciesTransport diffusion) backwards. fs, fa and gf are
+// the face state, aux and aux gradient (averages of the two cells); each side receives half of the adjoints
+// fsb (state), fab (T, u) and of the aux gradient's, which is made of one number per aux component and the
+// area normal n (aux_gradient_adjoint):
+//   T: -gs n,   u_c: -(gs_c n_d + gs_d n_c - 2/3 delta_cd gs.n),   Y_s: -gs n
 template <int DIM, int NS>
 __device__ __forceinline__ void diffusion_vjp(const Phys& P, const double* normal, const double* fs, const double* fa, const double* gf, bool dif,
-                                              bool spdif, const double* fb, double* fsb, double* fab, double* gfb) {
+                                              bool spdif, const double* fb, double* fsb, double* fab, double* gs) {
     using D = Dims<DIM, NS>;
 ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NC; k++) fsb[k] = 0.0;
 ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NA; k++) fab[k] = 0.0;
-ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NA * DIM; k++) gfb[k] = 0.0;
+    for (int k = 0; k < D::NA; k++) gs[k] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 1 + DIM; k++) fab[k] = 0.0;
     double mu, kc, diff;
     transport<DIM, NS>(P, NS, fs, fa[0], &mu, &kc, &diff);
     double mub = 0, kb = 0, Db = 0;
@@ -573,43 +576,19 @@ ABL_UNROLL_SPECIES
         double divVel = 0;
 #pragma unroll
         for (int c = 0; c < DIM; ++c) divVel += gv[c * DIM + c];
-        double tau[DIM * DIM], taub[DIM * DIM];
 #pragma unroll
-        for (int c = 0; c < DIM; ++c)
+        for (int c = 0; c < DIM; ++c) {
+            double sn = 0;  // row c of the stress over mu, times n
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) {
-                tau[c * DIM + d] = (d == c) ? 2.0 * mu * (gv[c * DIM + d] - divVel / 3.0) : mu * (gv[c * DIM + d] + gv[d * DIM + c]);
-                taub[c * DIM + d] = -normal[d] * fb[2 + c];
-            }
-        // energy: -sum_d n_d (sum_c u_c tau_dc + k dT/dx_d)
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-#pragma unroll
-            for (int c = 0; c < DIM; ++c) {
-                taub[d * DIM + c] -= normal[d] * fa[1 + c] * fb[1];
-                fab[1 + c] -= normal[d] * tau[d * DIM + c] * fb[1];
-            }
-            kb -= normal[d] * gT[d] * fb[1];
-            gfb[d] -= normal[d] * kc * fb[1];
+            for (int d = 0; d < DIM; ++d)
+                sn += ((d == c) ? 2.0 * (gv[c * DIM + c] - divVel / 3.0) : gv[c * DIM + d] + gv[d * DIM + c]) * normal[d];
+            const double w = fb[2 + c] + fa[1 + c] * fb[1];
+            fab[1 + c] = -mu * sn * fb[1];
+            mub -= w * sn;
+            gs[1 + c] = mu * w;
+            kb -= normal[c] * gT[c] * fb[1];
         }
-        double divb = 0;
-#pragma unroll
-        for (int c = 0; c < DIM; ++c)
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) {
-                const double tb = taub[c * DIM + d];
-                if (c == d) {
-                    gfb[DIM + c * DIM + c] += 2.0 * mu * tb;
-                    divb -= 2.0 * mu / 3.0 * tb;
-                    mub += 2.0 * tb * (gv[c * DIM + c] - divVel / 3.0);
-                } else {
-                    gfb[DIM + c * DIM + d] += mu * tb;
-                    gfb[DIM + d * DIM + c] += mu * tb;
-                    mub += tb * (gv[c * DIM + d] + gv[d * DIM + c]);
-                }
-            }
-#pragma unroll
-        for (int c = 0; c < DIM; ++c) gfb[DIM + c * DIM + c] += divb;
+        gs[0] = kc * fb[1];
     }
     if constexpr (NS > 0) {
         if (spdif) {
@@ -628,17 +607,14 @@ ABL_UNROLL_SPECIES
                 }
                 // one constant D_k per species (no state dependence), or the transport model's D
                 const double Ds = P.diff_k ? P.diff_k[s] : diff;
-                double hsb = 0;
+                double gn = 0;
 #pragma unroll
-                for (int d = 0; d < DIM; ++d) {
-                    const double gy = gf[yoff + s * DIM + d];
-                    const double q = -normal[d] * (fb[D::NE + s] + hs * fb[1]);
-                    rhob += q * Ds * gy;
-                    if (!P.diff_k) Db += q * density * gy;
-                    gfb[yoff + s * DIM + d] += q * density * Ds;
-                    hsb -= normal[d] * density * Ds * gy * fb[1];
-                }
-                Tb += hsb * cps;
+                for (int d = 0; d < DIM; ++d) gn += normal[d] * gf[yoff + s * DIM + d];
+                const double q = fb[D::NE + s] + hs * fb[1];
+                rhob -= q * Ds * gn;
+                if (!P.diff_k) Db -= q * density * gn;
+                gs[1 + DIM + s] = q * density * Ds;
+                Tb -= density * Ds * gn * fb[1] * cps;
             }
             fsb[0] += rhob;
             fab[0] += Tb;
@@ -647,126 +623,61 @@ ABL_UNROLL_SPECIES
     transport_vjp<DIM, NS>(P, NS, fs, fa[0], mub, kb, Db, fsb, &fab[0]);
 }
 
+// ga += half of the aux gradient's adjoint of a face with area normal n (see diffusion_vjp)
+template <int DIM, int NS>
+__device__ __forceinline__ void aux_gradient_adjoint(const double* n, const double* gs, double* ga) {
+    using D = Dims<DIM, NS>;
+    double tr = 0;
+#pragma unroll
+    for (int d = 0; d < DIM; d++) {
+        ga[d] -= 0.5 * gs[0] * n[d];
+        tr += gs[1 + d] * n[d];
+    }
+#pragma unroll
+    for (int c = 0; c < DIM; c++)
+#pragma unroll
+        for (int d = 0; d < DIM; d++) ga[(1 + c) * DIM + d] -= 0.5 * (gs[1 + c] * n[d] + gs[1 + d] * n[c] - (c == d ? 2.0 / 3.0 * tr : 0.0));
+ABL_UNROLL_SPECIES
+    for (int s = 0; s < NS; s++)
+#pragma unroll
+        for (int d = 0; d < DIM; d++) ga[(1 + DIM + s) * DIM + d] -= 0.5 * gs[1 + DIM + s] * n[d];
+}
+
 // ---------------------------------------------------------------------------------------------------
-// per-cell accumulators: [state NC][limited gradient NC*DIM][aux NA][aux gradient NA*DIM]
+// the adjoint row of a non-owned cell's side of one face: [state NC][limited gradient NC*DIM][aux NA][aux gradient NA*DIM]
 template <int DIM, int NS>
 struct AdjRow {
     using D = Dims<DIM, NS>;
     static constexpr int U = 0, G = D::NC, A = D::NC + D::NC * DIM, GA = D::NC + D::NC * DIM + D::NA;
     static constexpr int N = GA + D::NA * DIM;
-    static constexpr int S = N | 1;  // shared-memory row stride: odd, so rows of random cells spread over the banks
+    // shared-memory record of one face, [comp][face of the tile]: the diffusion pass leaves gs (NA), fab
+    // (1+DIM) and fsb's density and species (1+NS; its others are 0), the advection pass ubL and ubR
+    static constexpr int FG = 0, FA = D::NA, FS = D::NA + 1 + DIM;
+    static constexpr int R = FS + 1 + NS > 2 * D::NC ? FS + 1 + NS : 2 * D::NC;
 };
 
-// one face backwards, this lane's side: the adjoint contributions are added into the side's
-// accumulator row dst (nullptr drops a side that another tile accumulates)
-template <int DIM, int NS, int FK>
-__device__ __forceinline__ void face_vjp_side(const DevMesh& M, const Phys& P, unsigned mask, int side, int me, const double* normal,
-                                              const double* fdxo, const double* __restrict__ U, const double* __restrict__ aux,
-                                              const double* __restrict__ grad, const double* __restrict__ agrad, const double* __restrict__ Fb,
-                                              double* dst, bool* ok, bool* rok) {
+// dF_L/dflux = -1/V_L, dF_R/dflux = +1/V_R on owned cells: the flux adjoint of a face
+template <int DIM, int NS>
+__device__ __forceinline__ void flux_adjoint(const DevMesh& M, int2 lr, const double* __restrict__ Fb, double* fb) {
     using D = Dims<DIM, NS>;
-    using GR = GradRows<DIM, NS, double>;
-    using AR = AdjRow<DIM, NS>;
-    // dF_L/dflux = -1/V_L, dF_R/dflux = +1/V_R on owned cells; fb = (right term) + (left term)
-    const bool own = M.kind[me] == ABL_CELL_OWNED;
-    const double iv = own ? M.ivol[me] : 0.0;
-    double fb[D::NC];
+    const double iL = M.kind[lr.x] == ABL_CELL_OWNED ? -M.ivol[lr.x] : 0.0;
+    const double iR = M.kind[lr.y] == ABL_CELL_OWNED ? M.ivol[lr.y] : 0.0;
 ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NC; k++) {
-        const double t = own ? __ldg(Fb + (size_t)me * D::NC + k) * iv : 0.0;
-        const double mine = side ? t : -t;
-        fb[k] = mine + xch(mask, mine);
+        // a non-owned row of Fbar is not read: it may hold anything
+        const double l = iL != 0.0 ? __ldg(Fb + (size_t)lr.x * D::NC + k) * iL : 0.0;
+        const double r = iR != 0.0 ? __ldg(Fb + (size_t)lr.y * D::NC + k) * iR : 0.0;
+        fb[k] = l + r;
     }
-    double c[D::NC];
-    load_state<DIM, NS>(U, me, c);
-    const bool adv = P.advection && P.flux != ABL_FLUX_OFF;
-    const bool spadv = NS > 0 && P.sp_adv && P.flux != ABL_FLUX_OFF;
-    if (adv || spadv) {
-        const bool lsq = P.recon == ABL_RECON_LEASTSQUARES;
-        double u[D::NC];
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) {
-            double dot = 0;
-            if (lsq) {
-#pragma unroll
-                for (int d = 0; d < DIM; d++) dot += __ldg(grad + (size_t)me * GR::GS + k * DIM + d) * fdxo[d];
-            }
-            u[k] = lsq ? c[k] + dot : c[k];
-        }
-        double guess = 300.0;
-        if (NS > 0 && P.eos == ABL_EOS_NASA7) {
-            const double Tme = __ldg(aux + (size_t)me * D::NA), To = xch(mask, Tme);
-            const double TL = side ? To : Tme, TR = side ? Tme : To;
-            guess = side ? TL * .33 + .67 * TR : TL * .67 + .33 * TR;
-        }
-        double ub[D::NC];
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) ub[k] = 0.0;
-        advection_vjp_side<DIM, NS, FK>(P, mask, side, normal, u, guess, adv, spadv, fb, ub, ok, rok);
-        // u_face = u_cell + g . dx: the identity part to the state, the outer product with dx to the gradient
-        if (dst) {
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NC; k++) {
-                dst[AR::U + k] += ub[k];
-                if (lsq)
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) dst[AR::G + k * DIM + d] += ub[k] * fdxo[d];
-            }
-        }
-    }
-    const bool dif = P.diffusion && P.transport != ABL_TRANSPORT_NONE;
-    const bool spdif = NS > 0 && P.sp_dif && P.transport != ABL_TRANSPORT_NONE;
-    if (dif || spdif) {
-        // face averages: a + b is commutative, so both lanes hold identical values
-        double fs[D::NC], fa[D::NA], gf[D::NA * DIM];
-        {
-            double a[D::NA];
-            cell_aux<DIM, NS>(P, c, aux, me, a);
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NA; k++) fa[k] = a[k] * 0.5 + xch(mask, a[k]) * 0.5;
-        }
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) fs[k] = c[k] * 0.5 + xch(mask, c[k]) * 0.5;
-        // the face gradient: in 1D the two-cell LeastSquares stencil's (w_L a_L + w_R a_R, the same sum
-        // in both lanes), else the average of the two cells' aux gradients
-        double wme = 0.0;
-        if constexpr (DIM == 1) {
-            const double xme = fdxo[0], xot = xch(mask, fdxo[0]);  // each lane holds its side's offset
-            const double fdx2[6] = {side ? xot : xme, 0.0, 0.0, side ? xme : xot, 0.0, 0.0};
-            double wl, wr;
-            face_weights_1d(fdx2, &wl, &wr);
-            wme = side ? wr : wl;
-            const double wot = side ? wl : wr;
-            double a[D::NA];
-            cell_aux<DIM, NS>(P, c, aux, me, a);
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NA; k++) {
-                const double mine = a[k] * wme, other = xch(mask, a[k]) * wot;
-                gf[k] = side ? other + mine : mine + other;
-            }
-        } else {
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NA * DIM; k++) {
-                const double gm = __ldg(agrad + (size_t)me * GR::AS + k);
-                gf[k] = 0.5 * gm + 0.5 * xch(mask, gm);
-            }
-        }
-        double fsb[D::NC], fab[D::NA], gfb[D::NA * DIM];
-        diffusion_vjp<DIM, NS>(P, normal, fs, fa, gf, dif, spdif, fb, fsb, fab, gfb);
-        if (dst) {
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NC; k++) dst[AR::U + k] += 0.5 * fsb[k];
-            if constexpr (DIM == 1) {
-ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NA; k++) dst[AR::A + k] += 0.5 * fab[k] + wme * gfb[k];
-            } else {
-ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NA; k++) dst[AR::A + k] += 0.5 * fab[k];
-ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NA * DIM; k++) dst[AR::GA + k] += 0.5 * gfb[k];
-            }
-        }
-    }
+}
+
+// the record of the face's non-owned side in nbrec, or null: *side is that side
+template <int DIM, int NS>
+__device__ __forceinline__ double* nonowned_row(const DevMesh& M, int i, int2 lr, double* nbrec, int* side) {
+    const int nb = M.tf_nb[i];
+    if (nb < 0) return nullptr;
+    *side = M.kind[lr.x] != ABL_CELL_OWNED ? 0 : 1;
+    return nbrec + (size_t)nb * AdjRow<DIM, NS>::N;
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -790,59 +701,59 @@ struct GradRec {
     const int* ist;
 };
 
+// the state's part: ub and gt are the adjoints of the cell's state and limited gradient from its faces
 template <int DIM, int NS, int LIM>
-__device__ __forceinline__ void cell_vjp(const DevMesh& M, const Phys& P, int c, const double* __restrict__ U, const double* acc,
-                                         const GradRec& rec, const AdjOut<DIM, NS>& out, bool do_state, bool do_aux) {
+__device__ __forceinline__ void cell_vjp_state(const DevMesh& M, const Phys& P, int c, const double* __restrict__ U, double* ub, const double* gt,
+                                               const GradRec& rec, const AdjOut<DIM, NS>& out, bool do_state) {
     using D = Dims<DIM, NS>;
     using GR = GradRows<DIM, NS, double>;
-    using AR = AdjRow<DIM, NS>;
     const uint8_t kind = M.kind[c];
-    double ub[D::NC], gbar[D::NC * DIM], beta[D::NC];
-    int fst[D::NC];
+    const bool state = do_state && (kind == ABL_CELL_OWNED || kind == ABL_CELL_HALO);
+    double gbar[D::NC * DIM];
 ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NC; k++) {
-        ub[k] = acc[AR::U + k];
-        beta[k] = 0.0;
-        fst[k] = -1;
-    }
-ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NC * DIM; k++) gbar[k] = 0.0;
-    if (do_state && (kind == ABL_CELL_OWNED || kind == ABL_CELL_HALO)) {
-        // g~ = phi g (0 when cancelled): g-bar = phi g~-bar, plus the limiter's own dependence on g and on
-        // the minimising neighbour through r = (u_n - u_c) / (2 g . dx)
-        const double* g = rec.graw + (size_t)c * GR::GS;
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) {
+        double beta = 0.0;
+        int fst = -1;
+#pragma unroll
+        for (int d = 0; d < DIM; d++) gbar[k * DIM + d] = 0.0;
+        if (state) {
+            // g~ = phi g (0 when cancelled): g-bar = phi g~-bar, plus the limiter's own dependence on g and on
+            // the minimising neighbour through r = (u_n - u_c) / (2 g . dx)
+            const double* g = rec.graw + (size_t)c * GR::GS + k * DIM;
             const double ph = __ldg(rec.phi + (size_t)c * D::NC + k);
             const int i = __ldg(rec.ist + (size_t)c * D::NC + k);
             double phib = 0;
 #pragma unroll
             for (int d = 0; d < DIM; d++) {
-                const double gt = acc[AR::G + k * DIM + d];
-                gbar[k * DIM + d] = ph * gt;
-                phib += gt * __ldg(g + k * DIM + d);
+                gbar[k * DIM + d] = ph * gt[k * DIM + d];
+                phib += gt[k * DIM + d] * __ldg(g + d);
             }
-            if (i < 0 || phib == 0.0) continue;
-            const int2 ce = M.cone[i];
-            const int f = ce.x, n = ce.y & kConeNbr, sc = (ce.y & kConeSide) ? 1 : 0;
-            double v[DIM], denom = 0;
+            if (i >= 0 && phib != 0.0) {
+                const int2 ce = M.cone[i];
+                const int f = ce.x, n = ce.y & kConeNbr, sc = (ce.y & kConeSide) ? 1 : 0;
+                double v[DIM], denom = 0;
 #pragma unroll
-            for (int d = 0; d < DIM; d++) {
-                v[d] = __ldg(M.fdx + 6 * (size_t)f + 3 * sc + d) - __ldg(M.fdx + 6 * (size_t)f + 3 * (1 - sc) + d);
-                denom += __ldg(g + k * DIM + d) * v[d];
+                for (int d = 0; d < DIM; d++) {
+                    v[d] = __ldg(M.fdx + 6 * (size_t)f + 3 * sc + d) - __ldg(M.fdx + 6 * (size_t)f + 3 * (1 - sc) + d);
+                    denom += __ldg(g + d) * v[d];
+                }
+                const double idn = rcp64(denom);
+                const double r = 0.5 * (__ldg(U + (size_t)n * D::NC + k) - __ldg(U + (size_t)c * D::NC + k)) * idn;
+                const double dl = limiter_k<LIM, Dual>(P.limiter, Dual(r, 1.0)).d;
+                const double rb = dl * phib;
+                if (rb != 0.0 && isfinite(rb) && isfinite(r)) {
+                    beta = 0.5 * rb * idn;  // d r / d (u_n - u_c) = 1 / (2 denom)
+                    fst = f;
+                    ub[k] -= beta;
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) gbar[k * DIM + d] -= r * rb * idn * v[d];  // d r / d denom = -r / denom
+                }
             }
-            const double idn = rcp64(denom);
-            const double r = 0.5 * (__ldg(U + (size_t)n * D::NC + k) - __ldg(U + (size_t)c * D::NC + k)) * idn;
-            const double dl = limiter_k<LIM, Dual>(P.limiter, Dual(r, 1.0)).d;
-            const double rb = dl * phib;
-            if (rb == 0.0 || !isfinite(rb) || !isfinite(r)) continue;
-            const double bk = 0.5 * rb * idn;  // d r / d (u_n - u_c) = 1 / (2 denom)
-            beta[k] = bk;
-            fst[k] = f;
-            ub[k] -= bk;
-#pragma unroll
-            for (int d = 0; d < DIM; d++) gbar[k * DIM + d] -= r * rb * idn * v[d];  // d r / d denom = -r / denom
         }
+        out.beta[(size_t)c * D::NC + k] = beta;
+        out.fstar[(size_t)c * D::NC + k] = fst;
+    }
+    if (state) {
         // g = sum_f w_f (u_n - u_c): the own-cell term, with the cell's summed weights
 #pragma unroll
         for (int d = 0; d < DIM; d++) {
@@ -851,35 +762,33 @@ ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NC; k++) ub[k] -= ws * gbar[k * DIM + d];
         }
     }
-    double ab[D::NA], gab[D::NA * DIM];
-ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NA; k++) ab[k] = acc[AR::A + k];
-    const bool auxg = do_aux && kind != ABL_CELL_HALO_OUTER;
-ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NA * DIM; k++) gab[k] = auxg ? acc[AR::GA + k] : 0.0;
-    if (auxg) {
-#pragma unroll
-        for (int d = 0; d < DIM; d++) {
-            const double ws = __ldg(M.wsum + 6 * (size_t)c + 3 + d);
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NA; k++) ab[k] -= ws * gab[k * DIM + d];
-        }
-    }
     if (out.gb) {
         double* o = out.gb + (size_t)c * GR::GS;
 ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NC * DIM; k++) o[k] = gbar[k];
     }
 ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NC; k++) {
-        out.beta[(size_t)c * D::NC + k] = beta[k];
-        out.fstar[(size_t)c * D::NC + k] = fst[k];
-        out.ub[(size_t)c * D::NC + k] = ub[k];
+    for (int k = 0; k < D::NC; k++) out.ub[(size_t)c * D::NC + k] = ub[k];
+}
+
+// the aux fields' part: ab and ga are the adjoints of the cell's aux and aux gradient from its faces
+template <int DIM, int NS>
+__device__ __forceinline__ void cell_vjp_aux(const DevMesh& M, int c, double* ab, const double* ga, const AdjOut<DIM, NS>& out, bool do_aux) {
+    using D = Dims<DIM, NS>;
+    using GR = GradRows<DIM, NS, double>;
+    const bool auxg = do_aux && M.kind[c] != ABL_CELL_HALO_OUTER;
+    if (auxg) {
+#pragma unroll
+        for (int d = 0; d < DIM; d++) {
+            const double ws = __ldg(M.wsum + 6 * (size_t)c + 3 + d);
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NA; k++) ab[k] -= ws * ga[k * DIM + d];
+        }
     }
     if (out.gab) {
         double* o = out.gab + (size_t)c * GR::AS;
 ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NA * DIM; k++) o[k] = gab[k];
+        for (int k = 0; k < D::NA * DIM; k++) o[k] = auxg ? ga[k] : 0.0;
     }
 ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NA; k++) out.ab[(size_t)c * D::NA + k] = ab[k];
@@ -888,58 +797,225 @@ ABL_UNROLL_SPECIES
 // ---------------------------------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------------------------------
-// resident CTAs per SM the register budget targets (shared memory holds 2 tiles of accumulators at
-// 0 species; one at the species counts)
+// most threads of a CTA, and the resident CTAs per SM that the register budget targets: 128 registers without
+// species, 168 with up to 5, 255 with more
 template <int NS>
 struct AdjBlocks {
-    static constexpr int tile = NS == 0 ? 2 : 1;
+    static constexpr int threads = NS == 0 ? 256 : 128;
+    static constexpr int tile = NS == 0 ? 2 : (NS > 5 ? 2 : 3);
 };
 
-// 256 threads: two lanes per face, one colour (at most 128 faces) per pass
+// One CTA per tile, one thread per face and then one per cell, as the forward pass: the faces' adjoints
+// go to one shared-memory record per face, and every cell sums its faces' records in ascending face order
+// in registers (no atomics, no ordering between the faces). The diffusion and the advection flux take one
+// such round each: a round's record is a third of both, and so are the live registers. Bound by the latency
+// of its loads and FP64 chains. Two lanes per face, both evaluating what couples the sides, with per-cell
+// accumulators in shared memory that the faces updated colour by colour, took 114 M warp instructions at
+// 64^3 cells; this takes 65 M, and a seventh of the shared-memory wavefronts.
 template <int DIM, int NS, int FK, int LIM>
-__global__ void __launch_bounds__(256, AdjBlocks<NS>::tile) k_tile_adjoint(DevMesh M, Phys P, const double* __restrict__ U, const double* __restrict__ aux,
+__global__ void __launch_bounds__(AdjBlocks<NS>::threads, AdjBlocks<NS>::tile) k_tile_adjoint(DevMesh M, Phys P, const double* __restrict__ U, const double* __restrict__ aux,
                                                                           const double* __restrict__ grad, const double* __restrict__ agrad,
                                                                           const double* __restrict__ Fb, GradRec rec, AdjOut<DIM, NS> out,
                                                                           double* __restrict__ nbrec, int do_state, int do_aux, int* status) {
+    using D = Dims<DIM, NS>;
+    using GR = GradRows<DIM, NS, double>;
     using AR = AdjRow<DIM, NS>;
-    extern __shared__ double sacc[];  // [tile cells][AR::S]
+    extern __shared__ double srec[];  // [AR::R][tile faces]
     const int t = blockIdx.x;
-    const int cb = M.tile_cell_ptr[t], nct = M.tile_cell_ptr[t + 1] - cb;
-    for (int i = threadIdx.x; i < nct * AR::S; i += blockDim.x) sacc[i] = 0.0;
-    __syncthreads();
+    const int cb = M.tile_cell_ptr[t], ce = M.tile_cell_ptr[t + 1];
+    const int fb = M.tile_face_ptr[t], fe = M.tile_face_ptr[t + 1], nf = fe - fb;
     bool ok = true, rok = true;
-    const int side = threadIdx.x & 1, pair = threadIdx.x >> 1;
-    const int base = M.col_base[t], ncol = M.col_base[t + 1] - base - 1;
-    const int fb = M.tile_face_ptr[t];
-    for (int q = 0; q < ncol; q++) {
-        const int qa = M.col_start[base + q] + pair;
-        const bool act = qa < M.col_start[base + q + 1];
-        const unsigned mask = __ballot_sync(0xffffffffu, act);  // both lanes of a face share act
-        if (act) {
-            const int i = fb + M.tf_adj[qa];  // the face record
+    const bool dif = P.diffusion && P.transport != ABL_TRANSPORT_NONE;
+    const bool spdif = NS > 0 && P.sp_dif && P.transport != ABL_TRANSPORT_NONE;
+    const bool adv = P.advection && P.flux != ABL_FLUX_OFF;
+    const bool spadv = NS > 0 && P.sp_adv && P.flux != ABL_FLUX_OFF;
+    const bool lsq = P.recon == ABL_RECON_LEASTSQUARES;
+    if (dif || spdif) {
+        for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
             const int2 lr = M.tf_cells[i];
-            const int me = side ? lr.y : lr.x;
-            double normal[DIM], fdxo[3];
-            const double* geo = M.tf_geo + 10 * geo_record(M, i);
+            double normal[DIM], fdx[6], flb[D::NC], fs[D::NC], fa[D::NA], gf[D::NA * DIM];
+            face_geometry<DIM, double>(M, i, normal, fdx);
+            flux_adjoint<DIM, NS>(M, lr, Fb, flb);
+            double wl = 0, wr = 0;
+            {
+                double cL[D::NC], cR[D::NC], aL[D::NA], aR[D::NA];
+                load_state<DIM, NS>(U, lr.x, cL);
+                load_state<DIM, NS>(U, lr.y, cR);
+                cell_aux<DIM, NS>(P, cL, aux, lr.x, aL);
+                cell_aux<DIM, NS>(P, cR, aux, lr.y, aR);
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NC; k++) fs[k] = cL[k] * 0.5 + cR[k] * 0.5;
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NA; k++) fa[k] = aL[k] * 0.5 + aR[k] * 0.5;
+                if constexpr (DIM == 1) {
+                    // in 1D the face gradient is the two-cell LeastSquares stencil's
+                    face_weights_1d(fdx, &wl, &wr);
+ABL_UNROLL_SPECIES
+                    for (int k = 0; k < D::NA; k++) gf[k] = aL[k] * wl + aR[k] * wr;
+                }
+            }
+            if constexpr (DIM > 1) {
+                double gL[D::NA * DIM], gR[D::NA * DIM];
+                load_row<D::NA * DIM, double>(agrad + (size_t)lr.x * GR::AS, gL);
+                load_row<D::NA * DIM, double>(agrad + (size_t)lr.y * GR::AS, gR);
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NA * DIM; k++) gf[k] = 0.5 * gL[k] + 0.5 * gR[k];
+            }
+            double fsb[D::NC], fab[1 + DIM], gs[D::NA];
+            diffusion_vjp<DIM, NS>(P, normal, fs, fa, gf, dif, spdif, flb, fsb, fab, gs);
+            double* r = srec + (i - fb);
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NA; k++) r[(AR::FG + k) * nf] = gs[k];
 #pragma unroll
-            for (int d = 0; d < DIM; d++) normal[d] = __ldg(geo + d);
+            for (int k = 0; k < 1 + DIM; k++) r[(AR::FA + k) * nf] = fab[k];
+            r[AR::FS * nf] = fsb[0];
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < NS; k++) r[(AR::FS + 1 + k) * nf] = fsb[D::NE + k];
+            int side;
+            if (double* nr = nonowned_row<DIM, NS>(M, i, lr, nbrec, &side)) {
+                double ga[D::NA * DIM];
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NA * DIM; k++) ga[k] = 0.0;
+                aux_gradient_adjoint<DIM, NS>(normal, gs, ga);
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NC; k++) nr[AR::U + k] = 0.5 * fsb[k];
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NA; k++) {
+                    nr[AR::A + k] = (k < 1 + DIM ? 0.5 * fab[k < 1 + DIM ? k : 0] : 0.0) + (DIM == 1 ? 2.0 * (side ? wr : wl) * ga[k] : 0.0);
 #pragma unroll
-            for (int d = 0; d < 3; d++) fdxo[d] = __ldg(geo + 3 + 3 * side + d);
-            // destination: this tile's accumulator, the record of a non-owned side, or none
-            const uint32_t slots = M.tf_slot[i];
-            const int slot = side ? int(slots >> 16) : int(slots & 0xffff);
-            const int nb = M.tf_nb[i];
-            double* dst = nullptr;
-            if (slot != 0xffff)
-                dst = sacc + (size_t)slot * AR::S;
-            else if (nb >= 0 && M.kind[me] != ABL_CELL_OWNED)
-                dst = nbrec + (size_t)nb * AR::N;
-            face_vjp_side<DIM, NS, FK>(M, P, mask, side, me, normal, fdxo, U, aux, grad, agrad, Fb, dst, &ok, &rok);
+                    for (int d = 0; d < DIM; d++) nr[AR::GA + k * DIM + d] = DIM == 1 ? 0.0 : ga[k * DIM + d];
+                }
+            }
+        }
+        __syncthreads();
+        for (int j = cb + threadIdx.x; j < ce; j += blockDim.x) {
+            const int c = M.tile_cells[j];
+            double ab[D::NA], ga[D::NA * DIM], ub[D::NC];
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NA; k++) ab[k] = 0.0;
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NA * DIM; k++) ga[k] = 0.0;
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NC; k++) ub[k] = 0.0;
+            for (int e = M.tc_fptr[j]; e < M.tc_fptr[j + 1]; e++) {
+                const uint16_t code = M.tc_face[e];
+                const int q = code & 0x7fff;
+                const double* r = srec + q;
+                double normal[DIM], fdx[6], gs[D::NA];
+                face_geometry<DIM, double>(M, fb + q, normal, fdx);
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NA; k++) gs[k] = r[(AR::FG + k) * nf];
+                if constexpr (DIM == 1) {
+                    double wl, wr;
+                    face_weights_1d(fdx, &wl, &wr);
+                    double g1[D::NA];
+ABL_UNROLL_SPECIES
+                    for (int k = 0; k < D::NA; k++) g1[k] = 0.0;
+                    aux_gradient_adjoint<DIM, NS>(normal, gs, g1);
+ABL_UNROLL_SPECIES
+                    for (int k = 0; k < D::NA; k++) ab[k] += 2.0 * ((code & 0x8000) ? wr : wl) * g1[k];
+                } else {
+                    aux_gradient_adjoint<DIM, NS>(normal, gs, ga);
+                }
+#pragma unroll
+                for (int k = 0; k < 1 + DIM; k++) ab[k] += 0.5 * r[(AR::FA + k) * nf];
+                ub[0] += 0.5 * r[AR::FS * nf];
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < NS; k++) ub[D::NE + k] += 0.5 * r[(AR::FS + 1 + k) * nf];
+            }
+            cell_vjp_aux<DIM, NS>(M, c, ab, ga, out, do_aux);
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NC; k++) out.ub[(size_t)c * D::NC + k] = ub[k];  // read back below, by the same thread
         }
         __syncthreads();
     }
-    for (int j = threadIdx.x; j < nct; j += blockDim.x)
-        cell_vjp<DIM, NS, LIM>(M, P, M.tile_cells[cb + j], U, sacc + (size_t)j * AR::S, rec, out, do_state, do_aux);
+    if (adv || spadv) {
+        for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
+            const int2 lr = M.tf_cells[i];
+            double normal[DIM], fdx[6], uL[D::NC], uR[D::NC], flb[D::NC];
+            face_geometry<DIM, double>(M, i, normal, fdx);
+            load_state<DIM, NS>(U, lr.x, uL);
+            load_state<DIM, NS>(U, lr.y, uR);
+            if (lsq) {
+                double gL[D::NC * DIM], gR[D::NC * DIM];
+                load_row<D::NC * DIM, double>(grad + (size_t)lr.x * GR::GS, gL);
+                load_row<D::NC * DIM, double>(grad + (size_t)lr.y * GR::GS, gR);
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NC; k++) {
+                    double dotL = 0, dotR = 0;
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) {
+                        dotL += gL[k * DIM + d] * fdx[d];
+                        dotR += gR[k * DIM + d] * fdx[3 + d];
+                    }
+                    uL[k] += dotL;
+                    uR[k] += dotR;
+                }
+            }
+            double gsL = 300.0, gsR = 300.0;
+            if (NS > 0 && P.eos == ABL_EOS_NASA7) {
+                const double TL = __ldg(aux + (size_t)lr.x * D::NA), TR = __ldg(aux + (size_t)lr.y * D::NA);
+                gsL = TL * .67 + .33 * TR;
+                gsR = TL * .33 + .67 * TR;
+            }
+            flux_adjoint<DIM, NS>(M, lr, Fb, flb);
+            double ubL[D::NC], ubR[D::NC];
+            advection_vjp<DIM, NS, FK>(P, normal, uL, uR, gsL, gsR, adv, spadv, flb, ubL, ubR, &ok, &rok);
+            double* r = srec + (i - fb);
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NC; k++) {
+                r[k * nf] = ubL[k];
+                r[(D::NC + k) * nf] = ubR[k];
+            }
+            int side;
+            if (double* nr = nonowned_row<DIM, NS>(M, i, lr, nbrec, &side)) {
+                const bool first = !(dif || spdif);
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NC; k++) {
+                    const double v = side ? ubR[k] : ubL[k];
+                    nr[AR::U + k] = first ? v : nr[AR::U + k] + v;
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) nr[AR::G + k * DIM + d] = lsq ? v * fdx[side ? 3 + d : d] : 0.0;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    for (int j = cb + threadIdx.x; j < ce; j += blockDim.x) {
+        const int c = M.tile_cells[j];
+        double ub[D::NC], gt[D::NC * DIM];
+ABL_UNROLL_SPECIES
+        for (int k = 0; k < D::NC; k++) ub[k] = (dif || spdif) ? out.ub[(size_t)c * D::NC + k] : 0.0;
+ABL_UNROLL_SPECIES
+        for (int k = 0; k < D::NC * DIM; k++) gt[k] = 0.0;
+        if (adv || spadv)
+            for (int e = M.tc_fptr[j]; e < M.tc_fptr[j + 1]; e++) {
+                const uint16_t code = M.tc_face[e];
+                const int q = code & 0x7fff, side = code >> 15;
+                const double* r = srec + side * D::NC * nf + q;
+                const double* geo = M.tf_geo + 10 * geo_record(M, fb + q) + 3 + 3 * side;
+                double dx[DIM];
+#pragma unroll
+                for (int d = 0; d < DIM; d++) dx[d] = lsq ? __ldg(geo + d) : 0.0;
+                // u_face = u_cell + g . dx: the identity part to the state, the outer product with dx to the gradient
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NC; k++) {
+                    const double v = r[k * nf];
+                    ub[k] += v;
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) gt[k * DIM + d] += v * dx[d];
+                }
+            }
+        cell_vjp_state<DIM, NS, LIM>(M, P, c, U, ub, gt, rec, out, do_state);
+        if (!(dif || spdif)) {
+            double ab[D::NA], ga[D::NA * DIM];
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NA; k++) ab[k] = 0.0;
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NA * DIM; k++) ga[k] = 0.0;
+            cell_vjp_aux<DIM, NS>(M, c, ab, ga, out, do_aux);
+        }
+    }
     if (!ok) atomicOr(status, kStatusEos);
     if (!rok) atomicOr(status, kStatusRiemann);
 }
@@ -961,7 +1037,8 @@ ABL_UNROLL_SPECIES
 ABL_UNROLL_SPECIES
         for (int k = 0; k < AR::N; k++) acc[k] += r[k];
     }
-    cell_vjp<DIM, NS, LIM>(M, P, c, U, acc, rec, out, do_state, do_aux);
+    cell_vjp_aux<DIM, NS>(M, c, acc + AR::A, acc + AR::GA, out, do_aux);
+    cell_vjp_state<DIM, NS, LIM>(M, P, c, U, acc + AR::U, acc + AR::G, rec, out, do_state);
 }
 
 template <int DIM, int NS>

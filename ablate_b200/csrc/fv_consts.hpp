@@ -23,10 +23,6 @@
 
 namespace abl {
 
-// Faces per colour in a tile (the adjoint kernel runs one colour per pass, two lanes per face, on
-// 2 * kColorCap threads).
-constexpr int kColorCap = 128;
-
 // Largest species count a physics descriptor may carry (the per-thread scratch of the EOS batch
 // kernels is sized by it; the largest capacity instance holds it).
 constexpr int kMaxSpecies = 128;

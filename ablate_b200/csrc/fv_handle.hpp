@@ -92,11 +92,9 @@ struct abl_fv {
     int n_geo_classes = 0;          // 0: one geometry record per tile face record
     abl::DevBuf<uint16_t> tc_face;
     int tile_smem = 0;
-    // adjoint: tile face colours and slots, non-owned records
-    abl::DevBuf<int> col_base, col_start, tf_nb, face_nb, nonowned;
-    abl::DevBuf<uint32_t> tf_slot;
-    abl::DevBuf<uint16_t> tf_adj;
-    int tile_max_cells = 0, n_nb = 0;
+    // adjoint: records of the faces with a non-owned side
+    abl::DevBuf<int> tf_nb, face_nb, nonowned;
+    int tile_max_faces = 0, tile_cells_max = 0, n_nb = 0;  // most faces of a tile, cells of a full tile
     // the fused one-pass RHS: per-tile ext cells and class tables; usable per gradient precision
     // (0: FP64, 1: mixed) when a tile's rows fit in shared memory
     abl::DevBuf<int> fz_ext_ptr, fz_ext, fz_tile_cls, fz_cls_off, fz_pool;

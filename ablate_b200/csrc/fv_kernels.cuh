@@ -46,11 +46,7 @@ struct DevMesh {
     const double* tf_geo;     // [ntf][10]: area normal (3), face centroid minus each side's centroid (6), pad
     const int* tc_fptr;
     const uint16_t* tc_face;
-    // adjoint: face colours per tile, tile-local slots, records of faces with a non-owned side
-    const int* col_base;
-    const int* col_start;
-    const uint32_t* tf_slot;
-    const uint16_t* tf_adj;  // per tile, the record of the k-th face in adjoint colour order
+    // adjoint: records of faces with a non-owned side
     const int* tf_nb;
     const int* face_nb;
     int n_nonowned;

@@ -237,8 +237,8 @@ void run_vjp(abl_fv* fv, const double* U, const double* Fb, double* Ub, cudaStre
     mark(fv, "k_tile_adjoint", s);
     if (fv->n_nb > 0) ABL_CUDA(cudaMemsetAsync(fv->adj_nb.p, 0, (size_t)fv->n_nb * AR::N * sizeof(double), s));
     if (M.n_tiles > 0) {
-        const size_t smem = (size_t)fv->tile_max_cells * AR::S * sizeof(double);
-        if (smem > 227 * 1024) throw AblError(ABL_ERR_UNSUPPORTED, "adjoint accumulators exceed shared memory for this species count");
+        const size_t smem = (size_t)fv->tile_max_faces * AR::R * sizeof(double);
+        if (smem > 227 * 1024) throw AblError(ABL_ERR_UNSUPPORTED, "adjoint face records exceed shared memory for this species count");
         // flux calculator and limiter fixed at compile time where a specialised kernel exists
         auto kern = k_tile_adjoint<DIM, NS, -1, -1>;
         if constexpr (kSpecialized<NS>) {
@@ -249,8 +249,8 @@ void run_vjp(abl_fv* fv, const double* U, const double* Fb, double* Ub, cudaStre
                 kern = k_tile_adjoint<DIM, NS, ABL_FLUX_AUSM, -1>;
         }
         ABL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        static_assert(2 * kColorCap == 256, "one colour per pass of the 256-thread adjoint CTA");
-        kern<<<M.n_tiles, 256, smem, s>>>(M, P, U, fv->aux.p, fv->grad64.p, fv->agrad64.p, Fb, rec, out, fv->adj_nb.p, ds, da, fv->status.p);
+        const int threads = std::min(AdjBlocks<NS>::threads, std::max(128, fv->tile_cells_max));
+        kern<<<M.n_tiles, threads, smem, s>>>(M, P, U, fv->aux.p, fv->grad64.p, fv->agrad64.p, Fb, rec, out, fv->adj_nb.p, ds, da, fv->status.p);
         check_launch();
     }
     mark(fv, "k_adjoint_nonowned", s);

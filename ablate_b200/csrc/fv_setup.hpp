@@ -191,11 +191,9 @@ inline void lsq_pinv(int n, int dim, const double* B, double* W) {
 // the face geometry copied into tile order so the kernel streams it, and for every tile cell the
 // (local face, side) pairs in ascending global face order.
 //
-// The face records of a tile are in ascending face order. For the adjoint they are also coloured so
-// that no two faces of one colour touch the same tile cell, and listed colour by colour (tf_adj,
-// col_start). The adjoint kernel accumulates per-cell sums in shared memory one colour at a time,
-// which needs no atomics and fixes the summation order. A face with a side that is not an owned cell (a boundary ghost or a partition
-// halo) is in exactly one tile; its contribution to that side goes to a per-face record (nb index).
+// The face records of a tile are in ascending face order. A face with a side that is not an owned cell (a
+// boundary ghost or a partition halo) is in exactly one tile; the adjoint's contribution to that side goes
+// to a per-face record (nb index).
 struct Tiles {
     int n_tiles = 0;
     int max_faces = 0;                    // largest per-tile face count (sizes shared memory)
@@ -208,14 +206,9 @@ struct Tiles {
     std::vector<double> tf_fdx;           // [ntf][6] face centroid minus each side's centroid
     std::vector<int32_t> tc_fptr;         // [n_owned+1] per tile cell into tc_face
     std::vector<uint16_t> tc_face;        // local face index | side << 15
-    std::vector<uint32_t> tf_slot;        // [ntf] tile-local slot of L | of R << 16 (0xffff: not a tile cell)
-    std::vector<uint16_t> tf_adj;         // [ntf] per tile, the record of its k-th face in adjoint colour order
     std::vector<int32_t> tf_nb;           // [ntf] record of the non-owned side, -1 if both sides are owned
-    std::vector<int32_t> col_base;        // [n_tiles+1] into col_start
-    std::vector<int32_t> col_start;       // per tile: first position (in tf_adj) of each adjoint colour, then the end
     std::vector<int32_t> face_nb;         // [n_faces] record index of faces with a non-owned side, else -1
     int n_nb = 0;                         // number of such records
-    int max_colors = 0;
 };
 
 inline uint64_t morton_spread(uint64_t x, int dim) {
@@ -264,7 +257,6 @@ inline Tiles build_tiles(const HostMesh& h, const abl_mesh_desc* m, int tile_cel
     std::vector<int32_t> faces;
     t.face_ptr.push_back(0);
     t.tc_fptr.assign(n + 1, 0);
-    t.col_base.push_back(0);
     std::vector<std::vector<uint16_t>> lists;
     t.face_nb.assign(h.n_faces, -1);
     for (int f : h.flux_faces)
@@ -284,7 +276,6 @@ inline Tiles build_tiles(const HostMesh& h, const abl_mesh_desc* m, int tile_cel
         lists.assign(ce - cb, {});
         // face records in global face order (the flux pass reads them in this order, neighbouring
         // threads on neighbouring faces: the fastest of the orders measured)
-        const int base = (int)(t.tf_cells.size() / 2);
         for (size_t i = 0; i < faces.size(); i++) {
             const int f = faces[i];
             const int L = h.face_cells[2 * f], R = h.face_cells[2 * f + 1];
@@ -293,48 +284,8 @@ inline Tiles build_tiles(const HostMesh& h, const abl_mesh_desc* m, int tile_cel
             t.tf_face.push_back(f);
             for (int d = 0; d < 3; d++) t.tf_normal.push_back(d < dim ? m->face_normal[3 * (size_t)f + d] : 0.0);
             for (int z = 0; z < 6; z++) t.tf_fdx.push_back(h.fdx[6 * (size_t)f + z]);
-            t.tf_slot.push_back((uint32_t)(local[L] >= 0 ? local[L] : 0xffff) | ((uint32_t)(local[R] >= 0 ? local[R] : 0xffff) << 16));
             t.tf_nb.push_back(t.face_nb[f]);
         }
-        // the adjoint's colouring: balanced greedy. With K colours allowed each face takes the
-        // least-filled colour free at both its cells; K starts at the bound ceil(faces / kColorCap) and
-        // grows until every face fits. On an 8x8x4 hex tile (896 faces) that is 8 passes of 112 faces
-        // where first-fit needs 12 (six of them part-empty), and every pass ends at a CTA barrier.
-        std::vector<int> bcol;
-        int nb_col = 0;
-        for (int K = std::max(1, ((int)faces.size() + kColorCap - 1) / kColorCap); K <= 64 && nb_col == 0; K++) {
-            std::vector<uint64_t> u2(ce - cb, 0);
-            std::vector<int> c2(K, 0);
-            bcol.assign(faces.size(), 0);
-            bool fits = true;
-            for (size_t i = 0; i < faces.size() && fits; i++) {
-                const int f = faces[i];
-                const int lL = local[h.face_cells[2 * f]], lR = local[h.face_cells[2 * f + 1]];
-                const uint64_t busy = (lL >= 0 ? u2[lL] : 0) | (lR >= 0 ? u2[lR] : 0);
-                int c = -1;
-                for (int k = 0; k < K; k++)
-                    if (!((busy >> k) & 1ull) && c2[k] < kColorCap && (c < 0 || c2[k] < c2[c])) c = k;
-                if (c < 0) fits = false;
-                else {
-                    bcol[i] = c;
-                    c2[c]++;
-                    if (lL >= 0) u2[lL] |= 1ull << c;
-                    if (lR >= 0) u2[lR] |= 1ull << c;
-                }
-            }
-            if (fits) nb_col = K;
-        }
-        if (nb_col == 0) throw std::invalid_argument("tile face colouring needs more than 64 colours");
-        t.max_colors = std::max(t.max_colors, nb_col);
-        std::vector<int> aorder(faces.size());
-        for (size_t i = 0; i < faces.size(); i++) aorder[i] = (int)i;
-        std::stable_sort(aorder.begin(), aorder.end(), [&](int a, int b) { return bcol[a] < bcol[b]; });
-        for (size_t q = 0; q < aorder.size(); q++) {
-            if (q == 0 || bcol[aorder[q - 1]] != bcol[aorder[q]]) t.col_start.push_back(base + (int)q);
-            t.tf_adj.push_back((uint16_t)aorder[q]);
-        }
-        t.col_start.push_back(base + (int)faces.size());
-        t.col_base.push_back((int)t.col_start.size());
         // per-cell lists in ascending global face order, pointing at the face records
         for (size_t i = 0; i < faces.size(); i++) {
             const int f = faces[i];
