@@ -242,6 +242,9 @@ int instance_for(int dim, int ns) {
     return -1;
 }
 
+// components of the aux gradient per cell (GradComps::A)
+size_t aux_grad_comps(const abl_fv* fv) { return (size_t)fv->dim + fv->dim * (fv->dim + 1) / 2 + fv->ns * fv->dim; }
+
 // ---- species padding ----------------------------------------------------------------------------
 // A count without an instance of its own runs in a larger one: its rows there are [euler | pad
 // zero-state species | the caller's species]. Padding species have zero NASA-7 rows, infinite molar
@@ -734,19 +737,21 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
             fv->grad_early.upload(ge.data(), ge.size());
             fv->grad_late.upload(gl.data(), gl.size());
         }
+        fv->mesh.gs = (size_t)round_up(fv->n_cells, 32);  // every component's array starts on a 128-byte line
         fv->aux.alloc((size_t)fv->n_cells * fv->naux);
+        if (fv->need_aux) fv->tmp.alloc(fv->n_cells);
         {
             std::vector<double> a0((size_t)fv->n_cells * fv->naux, 0.0);
             for (int c = 0; c < fv->n_cells; c++) a0[(size_t)c * fv->naux] = 300.0;  // temperature guess (TChem::TemperatureFunction uses 300 K)
             ABL_CUDA(cudaMemcpy(fv->aux.p, a0.data(), a0.size() * sizeof(double), cudaMemcpyHostToDevice));
         }
         if (lsq) {
-            fv->grad64.alloc((size_t)fv->n_cells * round_up(fv->nc * fv->dim, 2));
-            if (fv->ns == 0 || fv->mixed_species) fv->grad32.alloc((size_t)fv->n_cells * round_up(fv->nc * fv->dim, 4));
+            fv->grad64.alloc(fv->mesh.gs * fv->nc * fv->dim);
+            if (fv->ns == 0 || fv->mixed_species) fv->grad32.alloc(fv->mesh.gs * fv->nc * fv->dim);
         }
         if (dif) {
-            fv->agrad64.alloc((size_t)fv->n_cells * round_up(fv->naux * fv->dim, 2));
-            if (fv->ns == 0 || fv->mixed_species) fv->agrad32.alloc((size_t)fv->n_cells * round_up(fv->naux * fv->dim, 4));
+            fv->agrad64.alloc(fv->mesh.gs * aux_grad_comps(fv.get()));
+            if (fv->ns == 0 || fv->mixed_species) fv->agrad32.alloc(fv->mesh.gs * aux_grad_comps(fv.get()));
         }
         fv->status.alloc(1);
         fv->status.zero();
@@ -953,8 +958,8 @@ int abl_fv_jvp(abl_fv* fv, double time, const double* U_dev, const double* dU_de
         if (!fv || !U_dev || !dU_dev || !dF_dev) throw std::invalid_argument("abl_fv_jvp: NULL argument");
         ABL_CUDA(cudaSetDevice(fv->device));
         // value + tangent gradient pairs, allocated on first use
-        if (fv->need_state_grad && fv->gradD.n == 0) fv->gradD.alloc((size_t)fv->n_cells * fv->nc * fv->dim * 2);
-        if (fv->need_aux_grad && fv->agradD.n == 0) fv->agradD.alloc((size_t)fv->n_cells * fv->naux * fv->dim * 2);
+        if (fv->need_state_grad && fv->gradD.n == 0) fv->gradD.alloc(fv->mesh.gs * fv->nc * fv->dim * 2);
+        if (fv->need_aux_grad && fv->agradD.n == 0) fv->agradD.alloc(fv->mesh.gs * aux_grad_comps(fv) * 2);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         if (fv->pad == 0) {
             dispatch_jvp(fv, U_dev, dU_dev, F_dev, dF_dev, s);
@@ -998,17 +1003,18 @@ int abl_fv_vjp(abl_fv* fv, double time, const double* U_dev, const double* Fbar_
         // per-cell adjoint records, allocated on first use
         const size_t n = (size_t)fv->n_cells;
         if (fv->adj_ub.n == 0) {
-            if (fv->need_state_grad) fv->adj_gb.alloc(n * round_up(fv->nc * fv->dim, 2));
-            if (fv->need_aux_grad) fv->adj_gab.alloc(n * round_up(fv->naux * fv->dim, 2));
-            fv->adj_beta.alloc(n * fv->nc);
-            fv->adj_fstar.alloc(n * fv->nc);
-            fv->adj_ab.alloc(n * fv->naux);
+            const size_t gs = fv->mesh.gs;
+            if (fv->need_state_grad) fv->adj_gb.alloc(gs * fv->nc * fv->dim);
+            if (fv->need_aux_grad) fv->adj_gab.alloc(gs * aux_grad_comps(fv));
+            fv->adj_beta.alloc(gs * fv->nc);
+            fv->adj_fstar.alloc(gs * fv->nc);
+            fv->adj_ab.alloc(gs * fv->naux);
             fv->adj_nb.alloc((size_t)std::max(fv->n_nb, 1) * (fv->nc + fv->nc * fv->dim + fv->naux + fv->naux * fv->dim));
-            fv->adj_ub.alloc(n * fv->nc);
+            fv->adj_ub.alloc(gs * fv->nc);
             if (fv->need_state_grad) {
-                fv->adj_graw.alloc(n * round_up(fv->nc * fv->dim, 2));
-                fv->adj_phi.alloc(n * fv->nc);
-                fv->adj_ist.alloc(n * fv->nc);
+                fv->adj_graw.alloc(gs * fv->nc * fv->dim);
+                fv->adj_phi.alloc(gs * fv->nc);
+                fv->adj_ist.alloc(gs * fv->nc);
             }
         }
         cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -187,7 +187,7 @@ ABL_HD void transport_vjp(const Phys& P, int ns, const double* U, double T, doub
 
 // reverse of cell_aux(): aux = (T, u, Y) of a cell from its conserved state
 template <int DIM, int NS>
-__device__ __forceinline__ void cell_aux_vjp(const Phys& P, const double* u, const double* __restrict__ aux, int c, const double* ab, double* Ub) {
+__device__ __forceinline__ void cell_aux_vjp(const Phys& P, const double* u, const double* __restrict__ tmp, int c, const double* ab, double* Ub) {
     using D = Dims<DIM, NS>;
     const double irho = rcp64(u[0]);
     double irhob = 0;
@@ -208,7 +208,7 @@ ABL_UNROLL_SPECIES
         double ys[NY], ysb[NY];
         fill_y(NS, u[0], u + D::NE, ys);
         bool ok = true;
-        const double T = temperature<DIM, NS>(P, NS, u, __ldg(aux + (size_t)c * D::NA), &ok);
+        const double T = temperature<DIM, NS>(P, NS, u, __ldg(tmp + c), &ok);
 ABL_UNROLL_SPECIES
         for (int k = 0; k < NS; k++) ysb[k] = 0.0;
         nasa_temperature_vjp<DIM, NS>(P, NS, u, ys, T, ab[0], ysb, Ub);
@@ -555,12 +555,14 @@ ABL_UNROLL_SPECIES
 // diffusion (NavierStokesTransport::DiffusionFlux, SpeciesTransport diffusion) backwards. fs, fa and gf are
 // the face state, aux and aux gradient (averages of the two cells); each side receives half of the adjoints
 // fsb (state), fab (T, u) and of the aux gradient's, which is made of one number per aux component and the
-// area normal n (aux_gradient_adjoint):
-//   T: -gs n,   u_c: -(gs_c n_d + gs_d n_c - 2/3 delta_cd gs.n),   Y_s: -gs n
+// area normal n (aux_gradient_adjoint). gf and the gradient's adjoint hold the velocity part in the symmetric
+// form of GradComps; the adjoint of du_c/dx_d is that of du_d/dx_c:
+//   T: -gs n,   u_c, d: -(gs_c n_d + gs_d n_c - 2/3 delta_cd gs.n),   Y_s: -gs n
 template <int DIM, int NS>
 __device__ __forceinline__ void diffusion_vjp(const Phys& P, const double* normal, const double* fs, const double* fa, const double* gf, bool dif,
                                               bool spdif, const double* fb, double* fsb, double* fab, double* gs) {
     using D = Dims<DIM, NS>;
+    using GC = GradComps<DIM, NS>;
 ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NC; k++) fsb[k] = 0.0;
 ABL_UNROLL_SPECIES
@@ -571,29 +573,26 @@ ABL_UNROLL_SPECIES
     transport<DIM, NS>(P, NS, fs, fa[0], &mu, &kc, &diff);
     double mub = 0, kb = 0, Db = 0;
     if (dif) {
-        const double* gT = gf;
-        const double* gv = gf + DIM;
         double divVel = 0;
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) divVel += gv[c * DIM + c];
+        for (int c = 0; c < DIM; ++c) divVel += gf[GC::sym(c, c)];
 #pragma unroll
         for (int c = 0; c < DIM; ++c) {
             double sn = 0;  // row c of the stress over mu, times n
 #pragma unroll
             for (int d = 0; d < DIM; ++d)
-                sn += ((d == c) ? 2.0 * (gv[c * DIM + c] - divVel / 3.0) : gv[c * DIM + d] + gv[d * DIM + c]) * normal[d];
+                sn += ((d == c) ? 2.0 * (gf[GC::sym(c, c)] - divVel / 3.0) : gf[GC::sym(c, d)]) * normal[d];
             const double w = fb[2 + c] + fa[1 + c] * fb[1];
             fab[1 + c] = -mu * sn * fb[1];
             mub -= w * sn;
             gs[1 + c] = mu * w;
-            kb -= normal[c] * gT[c] * fb[1];
+            kb -= normal[c] * gf[c] * fb[1];
         }
         gs[0] = kc * fb[1];
     }
     if constexpr (NS > 0) {
         if (spdif) {
             const double density = fs[0];
-            const int yoff = (1 + DIM) * DIM;
             double rhob = 0, Tb = 0;
 ABL_UNROLL_SPECIES
             for (int s = 0; s < NS; ++s) {
@@ -609,7 +608,7 @@ ABL_UNROLL_SPECIES
                 const double Ds = P.diff_k ? P.diff_k[s] : diff;
                 double gn = 0;
 #pragma unroll
-                for (int d = 0; d < DIM; ++d) gn += normal[d] * gf[yoff + s * DIM + d];
+                for (int d = 0; d < DIM; ++d) gn += normal[d] * gf[GC::Y + s * DIM + d];
                 const double q = fb[D::NE + s] + hs * fb[1];
                 rhob -= q * Ds * gn;
                 if (!P.diff_k) Db -= q * density * gn;
@@ -626,7 +625,7 @@ ABL_UNROLL_SPECIES
 // ga += half of the aux gradient's adjoint of a face with area normal n (see diffusion_vjp)
 template <int DIM, int NS>
 __device__ __forceinline__ void aux_gradient_adjoint(const double* n, const double* gs, double* ga) {
-    using D = Dims<DIM, NS>;
+    using GC = GradComps<DIM, NS>;
     double tr = 0;
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
@@ -636,20 +635,35 @@ __device__ __forceinline__ void aux_gradient_adjoint(const double* n, const doub
 #pragma unroll
     for (int c = 0; c < DIM; c++)
 #pragma unroll
-        for (int d = 0; d < DIM; d++) ga[(1 + c) * DIM + d] -= 0.5 * (gs[1 + c] * n[d] + gs[1 + d] * n[c] - (c == d ? 2.0 / 3.0 * tr : 0.0));
+        for (int d = c; d < DIM; d++) ga[GC::sym(c, d)] -= 0.5 * (gs[1 + c] * n[d] + gs[1 + d] * n[c] - (c == d ? 2.0 / 3.0 * tr : 0.0));
 ABL_UNROLL_SPECIES
     for (int s = 0; s < NS; s++)
 #pragma unroll
-        for (int d = 0; d < DIM; d++) ga[(1 + DIM + s) * DIM + d] -= 0.5 * gs[1 + DIM + s] * n[d];
+        for (int d = 0; d < DIM; d++) ga[GC::Y + s * DIM + d] -= 0.5 * gs[1 + DIM + s] * n[d];
+}
+// ab += sign times the weights w contracted with the aux gradient's adjoint ga (the reverse of
+// sum_d w_d (a_n - a_c) for T, u and Y)
+template <int DIM, int NS>
+__device__ __forceinline__ void contract_aux(double sign, const double* w, const double* ga, double* ab) {
+    using GC = GradComps<DIM, NS>;
+#pragma unroll
+    for (int d = 0; d < DIM; d++) {
+        const double x = sign * w[d];
+        ab[0] += x * ga[d];
+#pragma unroll
+        for (int c = 0; c < DIM; c++) ab[1 + c] += x * ga[GC::sym(c, d)];
+ABL_UNROLL_SPECIES
+        for (int s = 0; s < NS; s++) ab[1 + DIM + s] += x * ga[GC::Y + s * DIM + d];
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------
-// the adjoint row of a non-owned cell's side of one face: [state NC][limited gradient NC*DIM][aux NA][aux gradient NA*DIM]
+// the adjoint row of a non-owned cell's side of one face: [state NC][limited gradient NC*DIM][aux NA][aux gradient GradComps::A]
 template <int DIM, int NS>
 struct AdjRow {
     using D = Dims<DIM, NS>;
     static constexpr int U = 0, G = D::NC, A = D::NC + D::NC * DIM, GA = D::NC + D::NC * DIM + D::NA;
-    static constexpr int N = GA + D::NA * DIM;
+    static constexpr int N = GA + GradComps<DIM, NS>::A;
     // shared-memory record of one face, [comp][face of the tile]: the diffusion pass leaves gs (NA), fab
     // (1+DIM) and fsb's density and species (1+NS; its others are 0), the advection pass ubL and ubR
     static constexpr int FG = 0, FA = D::NA, FS = D::NA + 1 + DIM;
@@ -684,13 +698,13 @@ __device__ __forceinline__ double* nonowned_row(const DevMesh& M, int i, int2 lr
 // cell step: limiter and least-squares gradient backwards (the limiter recomputed), aux-gradient self
 // term; writes the per-cell records the gather reads
 template <int DIM, int NS>
-struct AdjOut {
-    double* gb;     // [nc][GS] adjoint of the unlimited state gradient
-    double* beta;   // [nc][NC] limiter term for the minimising neighbour
-    int* fstar;     // [nc][NC] face of that neighbour, -1 for none
-    double* gab;    // [nc][AS] adjoint of the aux gradient
-    double* ub;     // [nc][NC] state adjoint, own terms
-    double* ab;     // [nc][NA] aux adjoint, own terms
+struct AdjOut {  // component by component, as the gradients: [comp][cell]
+    double* gb;     // adjoint of the unlimited state gradient
+    double* beta;   // limiter term for the minimising neighbour
+    int* fstar;     // face of that neighbour, -1 for none
+    double* gab;    // adjoint of the aux gradient
+    double* ub;     // state adjoint, own terms
+    double* ab;     // aux adjoint, own terms
 };
 
 // forward records of k_gradient<..., REC = true>: unlimited gradient, applied limiter factor, and the
@@ -706,7 +720,7 @@ template <int DIM, int NS, int LIM>
 __device__ __forceinline__ void cell_vjp_state(const DevMesh& M, const Phys& P, int c, const double* __restrict__ U, double* ub, const double* gt,
                                                const GradRec& rec, const AdjOut<DIM, NS>& out, bool do_state) {
     using D = Dims<DIM, NS>;
-    using GR = GradRows<DIM, NS, double>;
+    using GC = GradComps<DIM, NS>;
     const uint8_t kind = M.kind[c];
     const bool state = do_state && (kind == ABL_CELL_OWNED || kind == ABL_CELL_HALO);
     double gbar[D::NC * DIM];
@@ -719,14 +733,16 @@ ABL_UNROLL_SPECIES
         if (state) {
             // g~ = phi g (0 when cancelled): g-bar = phi g~-bar, plus the limiter's own dependence on g and on
             // the minimising neighbour through r = (u_n - u_c) / (2 g . dx)
-            const double* g = rec.graw + (size_t)c * GR::GS + k * DIM;
-            const double ph = __ldg(rec.phi + (size_t)c * D::NC + k);
-            const int i = __ldg(rec.ist + (size_t)c * D::NC + k);
+            double g[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; d++) g[d] = __ldg(rec.graw + (k * DIM + d) * M.gs + c);
+            const double ph = __ldg(rec.phi + k * M.gs + c);
+            const int i = __ldg(rec.ist + k * M.gs + c);
             double phib = 0;
 #pragma unroll
             for (int d = 0; d < DIM; d++) {
                 gbar[k * DIM + d] = ph * gt[k * DIM + d];
-                phib += gt[k * DIM + d] * __ldg(g + d);
+                phib += gt[k * DIM + d] * g[d];
             }
             if (i >= 0 && phib != 0.0) {
                 const int2 ce = M.cone[i];
@@ -735,7 +751,7 @@ ABL_UNROLL_SPECIES
 #pragma unroll
                 for (int d = 0; d < DIM; d++) {
                     v[d] = __ldg(M.fdx + 6 * (size_t)f + 3 * sc + d) - __ldg(M.fdx + 6 * (size_t)f + 3 * (1 - sc) + d);
-                    denom += __ldg(g + d) * v[d];
+                    denom += g[d] * v[d];
                 }
                 const double idn = rcp64(denom);
                 const double r = 0.5 * (__ldg(U + (size_t)n * D::NC + k) - __ldg(U + (size_t)c * D::NC + k)) * idn;
@@ -750,8 +766,8 @@ ABL_UNROLL_SPECIES
                 }
             }
         }
-        out.beta[(size_t)c * D::NC + k] = beta;
-        out.fstar[(size_t)c * D::NC + k] = fst;
+        out.beta[k * M.gs + c] = beta;
+        out.fstar[k * M.gs + c] = fst;
     }
     if (state) {
         // g = sum_f w_f (u_n - u_c): the own-cell term, with the cell's summed weights
@@ -762,36 +778,27 @@ ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NC; k++) ub[k] -= ws * gbar[k * DIM + d];
         }
     }
-    if (out.gb) {
-        double* o = out.gb + (size_t)c * GR::GS;
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC * DIM; k++) o[k] = gbar[k];
-    }
-ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NC; k++) out.ub[(size_t)c * D::NC + k] = ub[k];
+    if (out.gb) store_comps<GC::S>(out.gb, M.gs, c, gbar);
+    store_comps<D::NC>(out.ub, M.gs, c, ub);
 }
 
 // the aux fields' part: ab and ga are the adjoints of the cell's aux and aux gradient from its faces
 template <int DIM, int NS>
 __device__ __forceinline__ void cell_vjp_aux(const DevMesh& M, int c, double* ab, const double* ga, const AdjOut<DIM, NS>& out, bool do_aux) {
     using D = Dims<DIM, NS>;
-    using GR = GradRows<DIM, NS, double>;
+    using GC = GradComps<DIM, NS>;
     const bool auxg = do_aux && M.kind[c] != ABL_CELL_HALO_OUTER;
     if (auxg) {
+        double ws[DIM];
 #pragma unroll
-        for (int d = 0; d < DIM; d++) {
-            const double ws = __ldg(M.wsum + 6 * (size_t)c + 3 + d);
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NA; k++) ab[k] -= ws * ga[k * DIM + d];
-        }
+        for (int d = 0; d < DIM; d++) ws[d] = __ldg(M.wsum + 6 * (size_t)c + 3 + d);
+        contract_aux<DIM, NS>(-1.0, ws, ga, ab);
     }
     if (out.gab) {
-        double* o = out.gab + (size_t)c * GR::AS;
 ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NA * DIM; k++) o[k] = auxg ? ga[k] : 0.0;
+        for (int k = 0; k < GC::A; k++) out.gab[k * M.gs + c] = auxg ? ga[k] : 0.0;
     }
-ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NA; k++) out.ab[(size_t)c * D::NA + k] = ab[k];
+    store_comps<D::NA>(out.ab, M.gs, c, ab);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -813,12 +820,12 @@ struct AdjBlocks {
 // accumulators in shared memory that the faces updated colour by colour, took 114 M warp instructions at
 // 64^3 cells; this takes 65 M, and a seventh of the shared-memory wavefronts.
 template <int DIM, int NS, int FK, int LIM>
-__global__ void __launch_bounds__(AdjBlocks<NS>::threads, AdjBlocks<NS>::tile) k_tile_adjoint(DevMesh M, Phys P, const double* __restrict__ U, const double* __restrict__ aux,
+__global__ void __launch_bounds__(AdjBlocks<NS>::threads, AdjBlocks<NS>::tile) k_tile_adjoint(DevMesh M, Phys P, const double* __restrict__ U, const double* __restrict__ tmp,
                                                                           const double* __restrict__ grad, const double* __restrict__ agrad,
                                                                           const double* __restrict__ Fb, GradRec rec, AdjOut<DIM, NS> out,
                                                                           double* __restrict__ nbrec, int do_state, int do_aux, int* status) {
     using D = Dims<DIM, NS>;
-    using GR = GradRows<DIM, NS, double>;
+    using GC = GradComps<DIM, NS>;
     using AR = AdjRow<DIM, NS>;
     extern __shared__ double srec[];  // [AR::R][tile faces]
     const int t = blockIdx.x;
@@ -833,7 +840,7 @@ __global__ void __launch_bounds__(AdjBlocks<NS>::threads, AdjBlocks<NS>::tile) k
     if (dif || spdif) {
         for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
             const int2 lr = M.tf_cells[i];
-            double normal[DIM], fdx[6], flb[D::NC], fs[D::NC], fa[D::NA], gf[D::NA * DIM];
+            double normal[DIM], fdx[6], flb[D::NC], fs[D::NC], fa[D::NA], gf[GC::A];
             face_geometry<DIM, double>(M, i, normal, fdx);
             flux_adjoint<DIM, NS>(M, lr, Fb, flb);
             double wl = 0, wr = 0;
@@ -841,8 +848,8 @@ __global__ void __launch_bounds__(AdjBlocks<NS>::threads, AdjBlocks<NS>::tile) k
                 double cL[D::NC], cR[D::NC], aL[D::NA], aR[D::NA];
                 load_state<DIM, NS>(U, lr.x, cL);
                 load_state<DIM, NS>(U, lr.y, cR);
-                cell_aux<DIM, NS>(P, cL, aux, lr.x, aL);
-                cell_aux<DIM, NS>(P, cR, aux, lr.y, aR);
+                cell_aux<DIM, NS>(P, cL, tmp, lr.x, aL);
+                cell_aux<DIM, NS>(P, cR, tmp, lr.y, aR);
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NC; k++) fs[k] = cL[k] * 0.5 + cR[k] * 0.5;
 ABL_UNROLL_SPECIES
@@ -855,11 +862,11 @@ ABL_UNROLL_SPECIES
                 }
             }
             if constexpr (DIM > 1) {
-                double gL[D::NA * DIM], gR[D::NA * DIM];
-                load_row<D::NA * DIM, double>(agrad + (size_t)lr.x * GR::AS, gL);
-                load_row<D::NA * DIM, double>(agrad + (size_t)lr.y * GR::AS, gR);
+                double gL[GC::A], gR[GC::A];
+                load_comps<GC::A>(agrad, M.gs, lr.x, gL);
+                load_comps<GC::A>(agrad, M.gs, lr.y, gR);
 ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NA * DIM; k++) gf[k] = 0.5 * gL[k] + 0.5 * gR[k];
+                for (int k = 0; k < GC::A; k++) gf[k] = 0.5 * gL[k] + 0.5 * gR[k];
             }
             double fsb[D::NC], fab[1 + DIM], gs[D::NA];
             diffusion_vjp<DIM, NS>(P, normal, fs, fa, gf, dif, spdif, flb, fsb, fab, gs);
@@ -873,28 +880,27 @@ ABL_UNROLL_SPECIES
             for (int k = 0; k < NS; k++) r[(AR::FS + 1 + k) * nf] = fsb[D::NE + k];
             int side;
             if (double* nr = nonowned_row<DIM, NS>(M, i, lr, nbrec, &side)) {
-                double ga[D::NA * DIM];
+                double ga[GC::A];
 ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NA * DIM; k++) ga[k] = 0.0;
+                for (int k = 0; k < GC::A; k++) ga[k] = 0.0;
                 aux_gradient_adjoint<DIM, NS>(normal, gs, ga);
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NC; k++) nr[AR::U + k] = 0.5 * fsb[k];
 ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NA; k++) {
+                for (int k = 0; k < D::NA; k++)
                     nr[AR::A + k] = (k < 1 + DIM ? 0.5 * fab[k < 1 + DIM ? k : 0] : 0.0) + (DIM == 1 ? 2.0 * (side ? wr : wl) * ga[k] : 0.0);
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) nr[AR::GA + k * DIM + d] = DIM == 1 ? 0.0 : ga[k * DIM + d];
-                }
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < GC::A; k++) nr[AR::GA + k] = DIM == 1 ? 0.0 : ga[k];
             }
         }
         __syncthreads();
         for (int j = cb + threadIdx.x; j < ce; j += blockDim.x) {
             const int c = M.tile_cells[j];
-            double ab[D::NA], ga[D::NA * DIM], ub[D::NC];
+            double ab[D::NA], ga[GC::A], ub[D::NC];
 ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NA; k++) ab[k] = 0.0;
 ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NA * DIM; k++) ga[k] = 0.0;
+            for (int k = 0; k < GC::A; k++) ga[k] = 0.0;
 ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NC; k++) ub[k] = 0.0;
             for (int e = M.tc_fptr[j]; e < M.tc_fptr[j + 1]; e++) {
@@ -908,9 +914,9 @@ ABL_UNROLL_SPECIES
                 if constexpr (DIM == 1) {
                     double wl, wr;
                     face_weights_1d(fdx, &wl, &wr);
-                    double g1[D::NA];
+                    double g1[GC::A];  // (T, u, Y), as the aux components
 ABL_UNROLL_SPECIES
-                    for (int k = 0; k < D::NA; k++) g1[k] = 0.0;
+                    for (int k = 0; k < GC::A; k++) g1[k] = 0.0;
                     aux_gradient_adjoint<DIM, NS>(normal, gs, g1);
 ABL_UNROLL_SPECIES
                     for (int k = 0; k < D::NA; k++) ab[k] += 2.0 * ((code & 0x8000) ? wr : wl) * g1[k];
@@ -924,8 +930,7 @@ ABL_UNROLL_SPECIES
                 for (int k = 0; k < NS; k++) ub[D::NE + k] += 0.5 * r[(AR::FS + 1 + k) * nf];
             }
             cell_vjp_aux<DIM, NS>(M, c, ab, ga, out, do_aux);
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NC; k++) out.ub[(size_t)c * D::NC + k] = ub[k];  // read back below, by the same thread
+            store_comps<D::NC>(out.ub, M.gs, c, ub);  // read back below, by the same thread
         }
         __syncthreads();
     }
@@ -937,9 +942,9 @@ ABL_UNROLL_SPECIES
             load_state<DIM, NS>(U, lr.x, uL);
             load_state<DIM, NS>(U, lr.y, uR);
             if (lsq) {
-                double gL[D::NC * DIM], gR[D::NC * DIM];
-                load_row<D::NC * DIM, double>(grad + (size_t)lr.x * GR::GS, gL);
-                load_row<D::NC * DIM, double>(grad + (size_t)lr.y * GR::GS, gR);
+                double gL[GC::S], gR[GC::S];
+                load_comps<GC::S>(grad, M.gs, lr.x, gL);
+                load_comps<GC::S>(grad, M.gs, lr.y, gR);
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NC; k++) {
                     double dotL = 0, dotR = 0;
@@ -954,7 +959,7 @@ ABL_UNROLL_SPECIES
             }
             double gsL = 300.0, gsR = 300.0;
             if (NS > 0 && P.eos == ABL_EOS_NASA7) {
-                const double TL = __ldg(aux + (size_t)lr.x * D::NA), TR = __ldg(aux + (size_t)lr.y * D::NA);
+                const double TL = __ldg(tmp + lr.x), TR = __ldg(tmp + lr.y);
                 gsL = TL * .67 + .33 * TR;
                 gsR = TL * .33 + .67 * TR;
             }
@@ -985,7 +990,7 @@ ABL_UNROLL_SPECIES
         const int c = M.tile_cells[j];
         double ub[D::NC], gt[D::NC * DIM];
 ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) ub[k] = (dif || spdif) ? out.ub[(size_t)c * D::NC + k] : 0.0;
+        for (int k = 0; k < D::NC; k++) ub[k] = (dif || spdif) ? out.ub[k * M.gs + c] : 0.0;
 ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NC * DIM; k++) gt[k] = 0.0;
         if (adv || spadv)
@@ -1008,11 +1013,11 @@ ABL_UNROLL_SPECIES
             }
         cell_vjp_state<DIM, NS, LIM>(M, P, c, U, ub, gt, rec, out, do_state);
         if (!(dif || spdif)) {
-            double ab[D::NA], ga[D::NA * DIM];
+            double ab[D::NA], ga[GC::A];
 ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NA; k++) ab[k] = 0.0;
 ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NA * DIM; k++) ga[k] = 0.0;
+            for (int k = 0; k < GC::A; k++) ga[k] = 0.0;
             cell_vjp_aux<DIM, NS>(M, c, ab, ga, out, do_aux);
         }
     }
@@ -1042,17 +1047,17 @@ ABL_UNROLL_SPECIES
 }
 
 template <int DIM, int NS>
-__global__ void __launch_bounds__(128) k_adjoint_gather(DevMesh M, Phys P, const double* __restrict__ U, const double* __restrict__ aux,
+__global__ void __launch_bounds__(128) k_adjoint_gather(DevMesh M, Phys P, const double* __restrict__ U, const double* __restrict__ tmp,
                                                         AdjOut<DIM, NS> in, double* __restrict__ Ub, int do_state, int do_aux, int* status) {
     using D = Dims<DIM, NS>;
-    using GR = GradRows<DIM, NS, double>;
+    using GC = GradComps<DIM, NS>;
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M.n_cells) return;
     double ub[D::NC], ab[D::NA];
 ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NC; k++) ub[k] = in.ub[(size_t)m * D::NC + k];
+    for (int k = 0; k < D::NC; k++) ub[k] = __ldg(in.ub + k * M.gs + m);
 ABL_UNROLL_SPECIES
-    for (int k = 0; k < D::NA; k++) ab[k] = in.ab[(size_t)m * D::NA + k];
+    for (int k = 0; k < D::NA; k++) ab[k] = __ldg(in.ab + k * M.gs + m);
     const int beg = M.cone_ptr[m];
     const size_t wb = weight_base(M, m, beg);
 #pragma unroll 1
@@ -1063,8 +1068,8 @@ ABL_UNROLL_SPECIES
         cone_weights<DIM, double>(M.cwar, nullptr, wb + (size_t)(i - beg), w, wa);
         if (do_state) {
             if (!(ce.y & kConeBoundary)) {
-                double gn[D::NC * DIM];
-                load_row<D::NC * DIM, double>(in.gb + (size_t)n * GR::GS, gn);
+                double gn[GC::S];
+                load_comps<GC::S>(in.gb, M.gs, n, gn);
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NC; k++)
 #pragma unroll
@@ -1072,20 +1077,17 @@ ABL_UNROLL_SPECIES
             }
 ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NC; k++)
-                if (__ldg(in.fstar + (size_t)n * D::NC + k) == f) ub[k] += __ldg(in.beta + (size_t)n * D::NC + k);
+                if (__ldg(in.fstar + k * M.gs + n) == f) ub[k] += __ldg(in.beta + k * M.gs + n);
         }
         if (do_aux) {
-            double gn[D::NA * DIM];
-            load_row<D::NA * DIM, double>(in.gab + (size_t)n * GR::AS, gn);
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NA; k++)
-#pragma unroll
-                for (int d = 0; d < DIM; d++) ab[k] += wa[d] * gn[k * DIM + d];
+            double gn[GC::A];
+            load_comps<GC::A>(in.gab, M.gs, n, gn);
+            contract_aux<DIM, NS>(1.0, wa, gn, ab);
         }
     }
     double u[D::NC];
     load_state<DIM, NS>(U, m, u);
-    cell_aux_vjp<DIM, NS>(P, u, aux, m, ab, ub);
+    cell_aux_vjp<DIM, NS>(P, u, tmp, m, ab, ub);
     bool finite = true;
 ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NC; k++) {

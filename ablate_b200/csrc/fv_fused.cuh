@@ -47,6 +47,14 @@ __host__ __device__ inline size_t fused_smem_bytes(int dim, int nc, int naux, in
 }
 constexpr size_t kFusedSmemLimit = 227 * 1024;
 
+// Row strides of the staged gradients, padded to whole 16-byte vectors
+template <int DIM, int NS, class G>
+struct GradRows {
+    static constexpr int V = 16 / sizeof(G);  // elements per 16-byte vector
+    static constexpr int GS = ((Dims<DIM, NS>::NC * DIM + V - 1) / V) * V;
+    static constexpr int AS = ((Dims<DIM, NS>::NA * DIM + V - 1) / V) * V;
+};
+
 // The rows of the face flux from shared memory, by tile-local slot (the counterpart of GlobalRows).
 template <int DIM, int NS, class G>
 struct SharedRows {
@@ -96,7 +104,7 @@ ABL_UNROLL_SPECIES
         }
     }
     __device__ __forceinline__ void grad_row(int c, G* g) const { row<D::NC * DIM>(sG + (size_t)c * GW, g); }
-    __device__ __forceinline__ void agrad_row(int c, G* g) const { row<D::NA * DIM>(sG + (size_t)c * GW + GR::GS, g); }
+    __device__ __forceinline__ void agrad_row(int c, G* g) const { row<GradComps<DIM, NS>::A>(sG + (size_t)c * GW + GR::GS, g); }
 };
 
 // Limiter of one field (components k0..k1-1) of a gradient cell, neighbour states from shared memory:
@@ -198,10 +206,7 @@ ABL_UNROLL_SPECIES
 ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NC * DIM; k++) out[k] = g[k];
     }
-    if (do_aux) {
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NA * DIM; k++) out[GR::GS + k] = ga[k];
-    }
+    if (do_aux) pack_aux_gradient<DIM, NS>(ga, out + GR::GS);
 }
 
 // One CTA per tile, persistent over the tiles [t0, t1) (CTA b takes tiles t0 + b, t0 + b + gridDim.x, ...).

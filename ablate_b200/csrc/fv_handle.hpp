@@ -63,7 +63,6 @@ inline void check_launch() {
     if (e != cudaSuccess) throw AblError(ABL_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
 }
 
-// gradient rows are padded to whole 16-byte vectors (see GradRows in fv_kernels.cuh)
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
 }  // namespace abl
@@ -111,6 +110,7 @@ struct abl_fv {
     const char* mark_names[8] = {};
     // work buffers: aux, gradients (FP64, FP32, and value+tangent pairs for the tangent kernels)
     abl::DevBuf<double> aux;
+    abl::DevBuf<double> tmp;  // the mixture's temperatures of aux alone, which the face and gradient passes read
     abl::DevBuf<double> grad64, agrad64, gradD, agradD;
     abl::DevBuf<float> grad32, agrad32;
     abl::DevBuf<int> status;

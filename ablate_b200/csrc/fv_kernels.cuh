@@ -29,6 +29,7 @@ enum StatusBits : int { kStatusNaN = 1, kStatusEos = 2, kStatusRiemann = 4 };
 struct DevMesh {
     int dim, n_cells, n_faces, n_flux_faces;
     const int2* face_cells;
+    size_t gs;  // stride of one component of the per-cell gradient and adjoint arrays: n_cells, padded
     const uint8_t* kind;
     const int* cone_ptr;
     // cone entry of a cell: x = face, y = neighbour | side << 31 | (face touches a boundary ghost) << 30
@@ -126,13 +127,55 @@ struct Dims {
     static constexpr int NA = 1 + DIM + NS;  // aux components per cell (T, u, Y)
 };
 
-// Row strides of the per-cell gradient arrays, padded to whole 16-byte vectors
-template <int DIM, int NS, class G>
-struct GradRows {
-    static constexpr int V = 16 / sizeof(G);  // elements per 16-byte vector
-    static constexpr int GS = ((Dims<DIM, NS>::NC * DIM + V - 1) / V) * V;
-    static constexpr int AS = ((Dims<DIM, NS>::NA * DIM + V - 1) / V) * V;
+// Components of the per-cell gradient arrays. They are stored component by component, [comp][cell]: the
+// face pass is bound by the L1's wavefronts (77 % of its peak with one row per cell, at 26 % of the issue
+// slots), and lanes on neighbouring cells then share a 128-byte line per component, where rows of 128 bytes
+// gave every lane a line of its own. The velocity part of the aux gradient is kept in the symmetric form that
+// the stress needs: du_c/dx_c, and du_c/dx_d + du_d/dx_c for c < d.
+template <int DIM, int NS>
+struct GradComps {
+    static constexpr int S = Dims<DIM, NS>::NC * DIM;   // state: [component][direction]
+    static constexpr int V = DIM * (DIM + 1) / 2;
+    static constexpr int Y = DIM + V;                   // first species gradient
+    static constexpr int A = Y + NS * DIM;              // aux: T, the symmetric velocity part, the species
+    // place of the symmetric velocity entry (c, d)
+    static __host__ __device__ constexpr int sym(int c, int d) {
+        return c <= d ? DIM + c * DIM - c * (c - 1) / 2 + (d - c) : DIM + d * DIM - d * (d - 1) / 2 + (c - d);
+    }
 };
+
+// the n components of cell c, component stride gs
+template <int N, class G>
+__device__ __forceinline__ void load_comps(const G* __restrict__ p, size_t gs, int c, G* out) {
+ABL_UNROLL_SPECIES
+    for (int k = 0; k < N; k++) {
+        if constexpr (std::is_same<G, Dual>::value) {
+            const double2 v = __ldg(reinterpret_cast<const double2*>(p) + k * gs + c);
+            out[k] = Dual(v.x, v.y);
+        } else {
+            out[k] = __ldg(p + k * gs + c);
+        }
+    }
+}
+template <int N, class G>
+__device__ __forceinline__ void store_comps(G* __restrict__ p, size_t gs, int c, const G* v) {
+ABL_UNROLL_SPECIES
+    for (int k = 0; k < N; k++) p[k * gs + c] = v[k];
+}
+
+// the gradient ga of (T, u, Y), [component][direction], as the aux arrays keep it
+template <int DIM, int NS, class G>
+__device__ __forceinline__ void pack_aux_gradient(const G* ga, G* out) {
+    using GC = GradComps<DIM, NS>;
+#pragma unroll
+    for (int d = 0; d < DIM; d++) out[d] = ga[d];
+#pragma unroll
+    for (int c = 0; c < DIM; c++)
+#pragma unroll
+        for (int d = c; d < DIM; d++) out[GC::sym(c, d)] = c == d ? ga[(1 + c) * DIM + c] : ga[(1 + c) * DIM + d] + ga[(1 + d) * DIM + c];
+ABL_UNROLL_SPECIES
+    for (int k = 0; k < NS * DIM; k++) out[GC::Y + k] = ga[(1 + DIM) * DIM + k];
+}
 
 // minimum resident CTAs per SM for __launch_bounds__ (register budget per thread = 65536 / (128 * n)),
 // chosen by timing: on the 128^3 gas gradient FP64 4 / FP32 6, tile FP64 4 (no spills at 128
@@ -147,37 +190,6 @@ struct MinBlocks {
 constexpr int kConeSide = int(1u << 31);
 constexpr int kConeBoundary = 1 << 30;
 constexpr int kConeNbr = (1 << 30) - 1;
-
-// load n elements of a 16-byte-aligned row with vector loads
-template <int N, class G>
-__device__ __forceinline__ void load_row(const G* __restrict__ p, G* out) {
-    if constexpr (std::is_same<G, Dual>::value) {
-ABL_UNROLL_SPECIES
-        for (int i = 0; i < N; i++) {
-            const double2 v = __ldg(reinterpret_cast<const double2*>(p) + i);
-            out[i] = Dual(v.x, v.y);
-        }
-    } else if constexpr (sizeof(G) == 8) {
-ABL_UNROLL_SPECIES
-        for (int i = 0; i < N / 2; i++) {
-            const double2 v = __ldg(reinterpret_cast<const double2*>(p) + i);
-            out[2 * i] = v.x;
-            out[2 * i + 1] = v.y;
-        }
-        if constexpr (N % 2) out[N - 1] = __ldg(p + N - 1);
-    } else {
-ABL_UNROLL_SPECIES
-        for (int i = 0; i < N / 4; i++) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(p) + i);
-            out[4 * i] = v.x;
-            out[4 * i + 1] = v.y;
-            out[4 * i + 2] = v.z;
-            out[4 * i + 3] = v.w;
-        }
-ABL_UNROLL_SPECIES
-        for (int i = (N / 4) * 4; i < N; i++) out[i] = __ldg(p + i);
-    }
-}
 
 template <class G>
 __device__ __forceinline__ G big_value();
@@ -235,26 +247,25 @@ ABL_UNROLL_SPECIES
     for (int s = 0; s < NS; s++) a[1 + DIM + s] = u[D::NE + s] * irho;
 }
 
-// aux (T, u, Y) of one cell: from the resident aux array for the mixture EOS, recomputed from the
-// conserved state for a perfect gas (UpdateAuxTemperatureField / UpdateAuxVelocityField /
-// UpdateAuxMassFractionField: navierStokesTransport.cpp:534-558, speciesTransport.cpp:98-110)
+// aux (T, u, Y) of one cell from its conserved state (UpdateAuxTemperatureField / UpdateAuxVelocityField /
+// UpdateAuxMassFractionField: navierStokesTransport.cpp:534-558, speciesTransport.cpp:98-110); the mixture's
+// temperature from tmp, the per-cell temperatures that k_aux left (a tangent solves it again from there, for
+// its derivative by the implicit-function theorem)
 template <int DIM, int NS, class S>
-__device__ __forceinline__ void cell_aux(const Phys& P, const S* u, const double* __restrict__ aux, int c, S* a) {
+__device__ __forceinline__ void cell_aux(const Phys& P, const S* u, const double* __restrict__ tmp, int c, S* a) {
     using D = Dims<DIM, NS>;
     if (NS > 0 && P.eos == ABL_EOS_NASA7) {
         if constexpr (std::is_same<S, Dual>::value) {
-            // tangent: T from the state (its derivative by the implicit-function theorem), the resident T as guess
             bool ok = true;
-            a[0] = temperature<DIM, NS>(P, NS, u, __ldg(aux + (size_t)c * D::NA), &ok);
-            const S irho = rcp64(u[0]);
-#pragma unroll
-            for (int d = 0; d < DIM; d++) a[1 + d] = u[2 + d] * irho;
-ABL_UNROLL_SPECIES
-            for (int s = 0; s < NS; s++) a[1 + DIM + s] = u[D::NE + s] * irho;
+            a[0] = temperature<DIM, NS>(P, NS, u, __ldg(tmp + c), &ok);
         } else {
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NA; k++) a[k] = __ldg(aux + (size_t)c * D::NA + k);
+            a[0] = __ldg(tmp + c);
         }
+        const S irho = rcp64(u[0]);
+#pragma unroll
+        for (int d = 0; d < DIM; d++) a[1 + d] = u[2 + d] * irho;
+ABL_UNROLL_SPECIES
+        for (int s = 0; s < NS; s++) a[1 + DIM + s] = u[D::NE + s] * irho;
         return;
     }
     aux_from_state<DIM, NS>(P, u, a);
@@ -266,30 +277,31 @@ ABL_UNROLL_SPECIES
 // shared and the two paths agree bit for bit.
 template <int DIM, int NS, class G>
 struct GlobalRows {
-    using D = Dims<DIM, NS>;
-    using GR = GradRows<DIM, NS, G>;
+    using GC = GradComps<DIM, NS>;
     const double* __restrict__ U;
     const double* __restrict__ dU;
-    const double* __restrict__ aux;
+    const double* __restrict__ tmp;
     const G* __restrict__ grad;
     const G* __restrict__ agrad;
+    size_t gs;
     template <class S>
     __device__ __forceinline__ void state(int c, S* u) const {
         load_state<DIM, NS, S>(U, dU, c, u);
     }
-    __device__ __forceinline__ double temperature(int c) const { return __ldg(aux + (size_t)c * D::NA); }
+    __device__ __forceinline__ double temperature(int c) const { return __ldg(tmp + c); }
     template <class S>
     __device__ __forceinline__ void aux_of(const Phys& P, const S* u, int c, S* a) const {
-        cell_aux<DIM, NS>(P, u, aux, c, a);
+        cell_aux<DIM, NS>(P, u, tmp, c, a);
     }
-    __device__ __forceinline__ void grad_row(int c, G* g) const { load_row<D::NC * DIM, G>(grad + (size_t)c * GR::GS, g); }
-    __device__ __forceinline__ void agrad_row(int c, G* g) const { load_row<D::NA * DIM, G>(agrad + (size_t)c * GR::AS, g); }
+    __device__ __forceinline__ void grad_row(int c, G* g) const { load_comps<GC::S, G>(grad, gs, c, g); }
+    __device__ __forceinline__ void agrad_row(int c, G* g) const { load_comps<GC::A, G>(agrad, gs, c, g); }
 };
 
 // ---------------------------------------------------------------------------------------------------
 // cells: the listed cells only (n_list of them), or every cell when null
 template <int DIM, int NS>
-__global__ void __launch_bounds__(256) k_aux(DevMesh M, Phys P, const double* __restrict__ U, double* __restrict__ aux, int* status,
+__global__ void __launch_bounds__(256) k_aux(DevMesh M, Phys P, const double* __restrict__ U, double* __restrict__ aux,
+                                             double* __restrict__ tmp, int* status,
                                              const int* __restrict__ cells = nullptr, int n_list = 0) {
     using D = Dims<DIM, NS>;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -299,7 +311,9 @@ __global__ void __launch_bounds__(256) k_aux(DevMesh M, Phys P, const double* __
     load_state<DIM, NS>(U, c, u);
     double* a = aux + (size_t)c * D::NA;
     bool ok = true;
-    a[0] = temperature<DIM, NS>(P, NS, u, a[0], &ok);
+    const double T = temperature<DIM, NS>(P, NS, u, a[0], &ok);
+    a[0] = T;
+    if (tmp) tmp[c] = T;  // a perfect gas, whose passes recompute T, has no copy
     const double irho = rcp64(u[0]);
 #pragma unroll
     for (int d = 0; d < DIM; d++) a[1 + d] = u[2 + d] * irho;
@@ -389,14 +403,14 @@ ABL_UNROLL_SPECIES
 // a zero row, so the flux kernel projects every cell without a branch.
 template <int DIM, int NS, class G, int LIM, bool REC = false>
 __global__ void __launch_bounds__(128, MinBlocks<NS, G>::grad) k_gradient(DevMesh M, Phys P, const double* __restrict__ U,
-                                                                    const double* __restrict__ dU, const double* __restrict__ aux,
+                                                                    const double* __restrict__ dU, const double* __restrict__ tmp,
                                                                     G* __restrict__ grad, G* __restrict__ agrad, int do_state, int do_aux,
                                                                     int cache, G* __restrict__ graw = nullptr, double* __restrict__ rphi = nullptr,
                                                                     int* __restrict__ rist = nullptr, const int* __restrict__ cells = nullptr,
                                                                     int n_list = 0) {
     extern __shared__ __align__(16) unsigned char gsm[];
     using D = Dims<DIM, NS>;
-    using GR = GradRows<DIM, NS, G>;
+    using GC = GradComps<DIM, NS>;
     using S = StateOf<G>;
     // cells: the listed cells only (n_list of them), or every cell when null
     const int ci = blockIdx.x * blockDim.x + threadIdx.x;
@@ -407,10 +421,9 @@ __global__ void __launch_bounds__(128, MinBlocks<NS, G>::grad) k_gradient(DevMes
     const size_t wb = weight_base(M, c, beg);
     const bool state = do_state && (kind == ABL_CELL_OWNED || kind == ABL_CELL_HALO);
     const bool auxg = do_aux && kind != ABL_CELL_HALO_OUTER;
-    const bool nasa = NS > 0 && P.eos == ABL_EOS_NASA7;
     S uc[D::NC], ac[D::NA];
     load_state<DIM, NS, S>(U, dU, c, uc);
-    if (auxg) cell_aux<DIM, NS>(P, uc, aux, c, ac);
+    if (auxg) cell_aux<DIM, NS>(P, uc, tmp, c, ac);
     G g[D::NC * DIM], ga[D::NA * DIM];
 ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NC * DIM; k++) g[k] = G(0);
@@ -424,7 +437,7 @@ ABL_UNROLL_SPECIES
             const int2 ce = M.cone[i];
             const int n = ce.y & kConeNbr;
             S un[D::NC];
-            if (state || !nasa || std::is_same<S, Dual>::value) load_state<DIM, NS, S>(U, dU, n, un);
+            load_state<DIM, NS, S>(U, dU, n, un);
             if (sd) {
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NC; k++) sd[((i - beg) * D::NC + k) * blockDim.x + threadIdx.x] = G(un[k] - uc[k]);
@@ -441,7 +454,7 @@ ABL_UNROLL_SPECIES
             }
             if (auxg) {
                 S an[D::NA];
-                cell_aux<DIM, NS>(P, un, aux, n, an);
+                cell_aux<DIM, NS>(P, un, tmp, n, an);
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NA; k++) {
                     const G delta = G(an[k] - ac[k]);
@@ -459,11 +472,7 @@ ABL_UNROLL_SPECIES
                 ph[k] = 1.0;
                 is[k] = -1;
             }
-            if (do_state) {
-                G* o = graw + (size_t)c * GR::GS;
-ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NC * DIM; k++) o[k] = g[k];
-            }
+            if (do_state) store_comps<GC::S>(graw, M.gs, c, g);
             if (state && P.limiter != ABL_LIMITER_NONE) {
                 limit_field<DIM, NS, G, LIM, true>(M, P, beg, end, wb, U, dU, uc, g, 0, D::NE, ph, is, sd);
                 if (NS > 0) limit_field<DIM, NS, G, LIM, true>(M, P, beg, end, wb, U, dU, uc, g, D::NE, D::NC, ph, is, sd);
@@ -471,8 +480,8 @@ ABL_UNROLL_SPECIES
             if (do_state) {
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NC; k++) {
-                    rphi[(size_t)c * D::NC + k] = ph[k];
-                    rist[(size_t)c * D::NC + k] = is[k];
+                    rphi[k * M.gs + c] = ph[k];
+                    rist[k * M.gs + c] = is[k];
                 }
             }
         } else if (state && P.limiter != ABL_LIMITER_NONE) {
@@ -480,15 +489,11 @@ ABL_UNROLL_SPECIES
             if (NS > 0) limit_field<DIM, NS, G, LIM>(M, P, beg, end, wb, U, dU, uc, g, D::NE, D::NC, nullptr, nullptr, sd);
         }
     }
-    if (do_state) {
-        G* out = grad + (size_t)c * GR::GS;
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC * DIM; k++) out[k] = g[k];
-    }
+    if (do_state) store_comps<GC::S>(grad, M.gs, c, g);
     if (do_aux) {
-        G* out = agrad + (size_t)c * GR::AS;
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NA * DIM; k++) out[k] = ga[k];
+        G sa[GC::A];
+        pack_aux_gradient<DIM, NS>(ga, sa);
+        store_comps<GC::A>(agrad, M.gs, c, sa);
     }
 }
 
@@ -713,7 +718,8 @@ ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NC; k++) fs[k] = cL[k] * 0.5 + cR[k] * 0.5;
 ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NA; k++) fa[k] = aL[k] * 0.5 + aR[k] * 0.5;
-        G gL[D::NA * DIM], gR[D::NA * DIM];
+        using GC = GradComps<DIM, NS>;
+        G gL[GC::A], gR[GC::A];
         if constexpr (DIM == 1) {
             // in 1D the face gradient is the two-cell LeastSquares stencil's; both sides carry it, so
             // the averages below return it exactly
@@ -729,19 +735,19 @@ ABL_UNROLL_SPECIES
         transport<DIM, NS>(P, NS, fs, fa[0], &mu, &kc, &diff);
         if (dif) {
             // NavierStokesTransport::DiffusionFlux + CompressibleFlowComputeStressTensor (navierStokesTransport.cpp:454-532)
-            G gv[DIM * DIM];
+            G gv[GC::V];  // the symmetric velocity gradient
 #pragma unroll
-            for (int i = 0; i < DIM * DIM; i++) gv[i] = G(0.5) * gL[DIM + i] + G(0.5) * gR[DIM + i];
+            for (int i = 0; i < GC::V; i++) gv[i] = G(0.5) * gL[DIM + i] + G(0.5) * gR[DIM + i];
             G divVel = 0;
 #pragma unroll
-            for (int c = 0; c < DIM; ++c) divVel += gv[c * DIM + c];
+            for (int c = 0; c < DIM; ++c) divVel += gv[GC::sym(c, c) - DIM];
             G tau[DIM * DIM];
             const G gmu = static_cast<G>(mu);
 #pragma unroll
             for (int c = 0; c < DIM; ++c)
 #pragma unroll
                 for (int d = 0; d < DIM; ++d)
-                    tau[c * DIM + d] = (d == c) ? G(2.0) * gmu * (gv[c * DIM + d] - divVel / G(3.0)) : gmu * (gv[c * DIM + d] + gv[d * DIM + c]);
+                    tau[c * DIM + d] = (d == c) ? G(2.0) * gmu * (gv[GC::sym(c, c) - DIM] - divVel / G(3.0)) : gmu * gv[GC::sym(c, d) - DIM];
 #pragma unroll
             for (int c = 0; c < DIM; ++c) {
                 G vf = 0;
@@ -774,7 +780,7 @@ ABL_UNROLL_SPECIES
 ABL_UNROLL_SPECIES
                     for (int s = 0; s < NS; s++) hs[s] = 0.0;
                 }
-                const int yoff = (1 + DIM) * DIM;
+                const int yoff = GC::Y;
                 S ef = 0;
 ABL_UNROLL_SPECIES
                 for (int s = 0; s < NS; ++s) {
@@ -836,7 +842,7 @@ __device__ __forceinline__ void face_geometry(const DevMesh& M, int i, double* n
 // Phase 2: each tile cell sums -+flux of its faces in ascending face order, adds the sum / V and writes F once.
 template <int DIM, int NS, class G, int FK>
 __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMesh M, Phys P, const double* __restrict__ U,
-                                                                     const double* __restrict__ dU, const double* __restrict__ aux,
+                                                                     const double* __restrict__ dU, const double* __restrict__ tmp,
                                                                      const G* __restrict__ grad, const G* __restrict__ agrad,
                                                                      double* __restrict__ F, double* __restrict__ dF, int overwrite,
                                                                      int* status, int t0 = 0) {
@@ -847,7 +853,7 @@ __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMe
     const int t = t0 + blockIdx.x;
     const int fb = M.tile_face_ptr[t], fe = M.tile_face_ptr[t + 1];
     bool ok = true, rok = true;
-    const GlobalRows<DIM, NS, G> src{U, dU, aux, grad, agrad};
+    const GlobalRows<DIM, NS, G> src{U, dU, tmp, grad, agrad, M.gs};
     for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
         const int2 lr = M.tf_cells[i];
         double normal[DIM], fdx[6];

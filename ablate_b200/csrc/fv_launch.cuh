@@ -13,7 +13,7 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
     if (smem > 227 * 1024) throw AblError(ABL_ERR_UNSUPPORTED, "tile flux buffer exceeds shared memory for this species count");
     ABL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (!fv->pipe_active) {
-        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->aux.p, grad, agrad, F, dF, overwrite, fv->status.p, 0);
+        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->tmp.p, grad, agrad, F, dF, overwrite, fv->status.p, 0);
         check_launch();
         return;
     }
@@ -22,7 +22,7 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
     const int nch = fv->chunk_tile.empty() ? 0 : (int)fv->chunk_tile.size() - 1;
     if (nch == 0) {
         ABL_CUDA(cudaStreamWaitEvent(s, fv->ev_in[0], 0));
-        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->aux.p, grad, agrad, F, dF, overwrite, fv->status.p, 0);
+        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->tmp.p, grad, agrad, F, dF, overwrite, fv->status.p, 0);
         check_launch();
         return;
     }
@@ -30,7 +30,7 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
         const int ta = fv->chunk_tile[q], tb = fv->chunk_tile[q + 1];
         ABL_CUDA(cudaStreamWaitEvent(s, fv->ev_in[q], 0));
         if (tb > ta) {
-            kern<<<tb - ta, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->aux.p, grad, agrad, F, dF, overwrite, fv->status.p, ta);
+            kern<<<tb - ta, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->tmp.p, grad, agrad, F, dF, overwrite, fv->status.p, ta);
             check_launch();
         }
         ABL_CUDA(cudaEventRecord(fv->ev_chunk[q], s));
@@ -94,7 +94,7 @@ void launch_gradient(abl_fv* fv, const double* U, const double* dU, G* grad, G* 
     const abl::DevBuf<int>* list = fv->rhs_phase == 0 ? &fv->grad_early : fv->rhs_phase == 1 ? &fv->grad_late : nullptr;
     const int n = list ? (int)list->n : fv->mesh.n_cells;
     if (n == 0) return;
-    k_gradient<DIM, NS, G, LIM><<<blocks_for(n, 128), 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->aux.p, grad, agrad, fv->need_state_grad,
+    k_gradient<DIM, NS, G, LIM><<<blocks_for(n, 128), 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->tmp.p, grad, agrad, fv->need_state_grad,
                                                                    fv->need_aux_grad, smem > 0, nullptr, nullptr, nullptr, list ? list->p : nullptr, n);
     check_launch();
 }
@@ -105,7 +105,7 @@ void launch_aux(abl_fv* fv, const double* U, cudaStream_t s) {
     const abl::DevBuf<int>* list = fv->rhs_phase == 0 ? &fv->aux_early : fv->rhs_phase == 1 ? &fv->aux_late : nullptr;
     const int n = list ? (int)list->n : fv->mesh.n_cells;
     if (n == 0) return;
-    k_aux<DIM, NS><<<blocks_for(n, 256), 256, 0, s>>>(fv->mesh, fv->phys, U, fv->aux.p, fv->status.p, list ? list->p : nullptr, n);
+    k_aux<DIM, NS><<<blocks_for(n, 256), 256, 0, s>>>(fv->mesh, fv->phys, U, fv->aux.p, fv->tmp.p, fv->status.p, list ? list->p : nullptr, n);
     check_launch();
 }
 
@@ -182,7 +182,7 @@ void run_rhs(abl_fv* fv, const double* U, double* F, int precision, int overwrit
 
 template <int DIM, int NS>
 void run_aux(abl_fv* fv, const double* U, cudaStream_t s) {
-    k_aux<DIM, NS><<<blocks_for(fv->mesh.n_cells, 256), 256, 0, s>>>(fv->mesh, fv->phys, U, fv->aux.p, fv->status.p);
+    k_aux<DIM, NS><<<blocks_for(fv->mesh.n_cells, 256), 256, 0, s>>>(fv->mesh, fv->phys, U, fv->aux.p, fv->tmp.p, fv->status.p);
     check_launch();
 }
 
@@ -193,7 +193,7 @@ void run_jvp(abl_fv* fv, const double* U, const double* dU, double* F, double* d
     fv->n_marks = 0;
     if (fv->need_aux) {
         mark(fv, "k_aux", s);
-        k_aux<DIM, NS><<<blocks_for(M.n_cells, 256), 256, 0, s>>>(M, fv->phys, U, fv->aux.p, fv->status.p);
+        k_aux<DIM, NS><<<blocks_for(M.n_cells, 256), 256, 0, s>>>(M, fv->phys, U, fv->aux.p, fv->tmp.p, fv->status.p);
         check_launch();
     }
     Dual* grad = reinterpret_cast<Dual*>(fv->gradD.p);
@@ -217,7 +217,7 @@ void run_vjp(abl_fv* fv, const double* U, const double* Fb, double* Ub, cudaStre
     fv->n_marks = 0;
     if (fv->need_aux) {
         mark(fv, "k_aux", s);
-        k_aux<DIM, NS><<<blocks_for(M.n_cells, 256), 256, 0, s>>>(M, P, U, fv->aux.p, fv->status.p);
+        k_aux<DIM, NS><<<blocks_for(M.n_cells, 256), 256, 0, s>>>(M, P, U, fv->aux.p, fv->tmp.p, fv->status.p);
         check_launch();
     }
     GradRec rec{fv->adj_graw.p, fv->adj_phi.p, fv->adj_ist.p};
@@ -227,7 +227,7 @@ void run_vjp(abl_fv* fv, const double* U, const double* Fb, double* Ub, cudaStre
         if constexpr (kSpecialized<NS>)
             if (P.limiter == ABL_LIMITER_MINMOD) kern = k_gradient<DIM, NS, double, ABL_LIMITER_MINMOD, true>;
         const size_t smem = gradient_smem<DIM, NS, double>(fv);
-        kern<<<blocks_for(M.n_cells, 128), 128, smem, s>>>(M, P, U, nullptr, fv->aux.p, fv->grad64.p, fv->agrad64.p, fv->need_state_grad,
+        kern<<<blocks_for(M.n_cells, 128), 128, smem, s>>>(M, P, U, nullptr, fv->tmp.p, fv->grad64.p, fv->agrad64.p, fv->need_state_grad,
                                                           fv->need_aux_grad, smem > 0, fv->adj_graw.p, fv->adj_phi.p, fv->adj_ist.p, nullptr, 0);
         check_launch();
     }
@@ -250,7 +250,7 @@ void run_vjp(abl_fv* fv, const double* U, const double* Fb, double* Ub, cudaStre
         }
         ABL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const int threads = std::min(AdjBlocks<NS>::threads, std::max(128, fv->tile_cells_max));
-        kern<<<M.n_tiles, threads, smem, s>>>(M, P, U, fv->aux.p, fv->grad64.p, fv->agrad64.p, Fb, rec, out, fv->adj_nb.p, ds, da, fv->status.p);
+        kern<<<M.n_tiles, threads, smem, s>>>(M, P, U, fv->tmp.p, fv->grad64.p, fv->agrad64.p, Fb, rec, out, fv->adj_nb.p, ds, da, fv->status.p);
         check_launch();
     }
     mark(fv, "k_adjoint_nonowned", s);
@@ -259,7 +259,7 @@ void run_vjp(abl_fv* fv, const double* U, const double* Fb, double* Ub, cudaStre
         check_launch();
     }
     mark(fv, "k_adjoint_gather", s);
-    k_adjoint_gather<DIM, NS><<<blocks_for(M.n_cells, 128), 128, 0, s>>>(M, P, U, fv->aux.p, out, Ub, ds, da, fv->status.p);
+    k_adjoint_gather<DIM, NS><<<blocks_for(M.n_cells, 128), 128, 0, s>>>(M, P, U, fv->tmp.p, out, Ub, ds, da, fv->status.p);
     check_launch();
     mark(fv, "end", s);
 }
