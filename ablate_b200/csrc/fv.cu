@@ -958,6 +958,7 @@ int abl_fv_jvp(abl_fv* fv, double time, const double* U_dev, const double* dU_de
         if (!fv || !U_dev || !dU_dev || !dF_dev) throw std::invalid_argument("abl_fv_jvp: NULL argument");
         ABL_CUDA(cudaSetDevice(fv->device));
         // value + tangent gradient pairs, allocated on first use
+        if (fv->need_aux && fv->tmpD.n == 0) fv->tmpD.alloc((size_t)fv->n_cells * 2);
         if (fv->need_state_grad && fv->gradD.n == 0) fv->gradD.alloc(fv->mesh.gs * fv->nc * fv->dim * 2);
         if (fv->need_aux_grad && fv->agradD.n == 0) fv->agradD.alloc(fv->mesh.gs * aux_grad_comps(fv) * 2);
         cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -34,4 +34,10 @@ constexpr int kMaxSpecies = 128;
 template <int NS>
 constexpr bool kSpecialized = NS <= 9;
 
+// Instances whose loops over the state components are unrolled (the others are the capacity instances,
+// ABL_CAPACITY_TU). Where a kernel has a second form, the capacity instances keep the first: their run-time
+// loops have returned wrong values from forms that are exact in every unrolled instance.
+template <int NS>
+constexpr bool kUnrolled = NS <= 16;
+
 }  // namespace abl

@@ -110,7 +110,8 @@ struct abl_fv {
     const char* mark_names[8] = {};
     // work buffers: aux, gradients (FP64, FP32, and value+tangent pairs for the tangent kernels)
     abl::DevBuf<double> aux;
-    abl::DevBuf<double> tmp;  // the mixture's temperatures of aux alone, which the face and gradient passes read
+    abl::DevBuf<double> tmp;   // the mixture's temperatures of aux alone, which the face and gradient passes read
+    abl::DevBuf<double> tmpD;  // (T, dT) pairs for the tangent passes, allocated on the first JVP
     abl::DevBuf<double> grad64, agrad64, gradD, agradD;
     abl::DevBuf<float> grad32, agrad32;
     abl::DevBuf<int> status;

@@ -180,11 +180,12 @@ ABL_UNROLL_SPECIES
 // minimum resident CTAs per SM for __launch_bounds__ (register budget per thread = 65536 / (128 * n)),
 // chosen by timing: on the 128^3 gas gradient FP64 4 / FP32 6, tile FP64 4 (no spills at 128
 // registers) / FP32 5; with 3-5 species 3 (5 species: 2.7 % faster than 2), with more species 2 (9
-// species on tetrahedra: 3 is 14 % slower); the value+tangent pairs of the tangent kernels 1
+// species on tetrahedra: 3 is 14 % slower); the value+tangent pairs of the tangent kernels 3 without species
+// (168 registers; with one CTA's 250 the 64^3 channel's JVP took 342 us against 297) and 2 with
 template <int NS, class G>
 struct MinBlocks {
-    static constexpr int grad = std::is_same<G, Dual>::value ? 1 : (NS > 5 ? 2 : (NS > 0 ? 3 : (sizeof(G) == 8 ? 4 : 6)));
-    static constexpr int tile = std::is_same<G, Dual>::value ? 1 : (NS > 5 ? 2 : (NS > 2 ? 3 : (sizeof(G) == 8 ? 4 : 5)));
+    static constexpr int grad = std::is_same<G, Dual>::value ? (NS == 0 ? 3 : 2) : (NS > 5 ? 2 : (NS > 0 ? 3 : (sizeof(G) == 8 ? 4 : 6)));
+    static constexpr int tile = std::is_same<G, Dual>::value ? (NS == 0 ? 3 : 2) : (NS > 5 ? 2 : (NS > 2 ? 3 : (sizeof(G) == 8 ? 4 : 5)));
 };
 
 constexpr int kConeSide = int(1u << 31);
@@ -249,15 +250,14 @@ ABL_UNROLL_SPECIES
 
 // aux (T, u, Y) of one cell from its conserved state (UpdateAuxTemperatureField / UpdateAuxVelocityField /
 // UpdateAuxMassFractionField: navierStokesTransport.cpp:534-558, speciesTransport.cpp:98-110); the mixture's
-// temperature from tmp, the per-cell temperatures that k_aux left (a tangent solves it again from there, for
-// its derivative by the implicit-function theorem)
+// temperature from tmp, the per-cell temperatures that k_aux left (k_aux_tangent for a tangent: (T, dT) pairs)
 template <int DIM, int NS, class S>
 __device__ __forceinline__ void cell_aux(const Phys& P, const S* u, const double* __restrict__ tmp, int c, S* a) {
     using D = Dims<DIM, NS>;
     if (NS > 0 && P.eos == ABL_EOS_NASA7) {
         if constexpr (std::is_same<S, Dual>::value) {
-            bool ok = true;
-            a[0] = temperature<DIM, NS>(P, NS, u, __ldg(tmp + c), &ok);
+            const double2 t = __ldg(reinterpret_cast<const double2*>(tmp) + c);
+            a[0] = Dual(t.x, t.y);
         } else {
             a[0] = __ldg(tmp + c);
         }
@@ -288,7 +288,7 @@ struct GlobalRows {
     __device__ __forceinline__ void state(int c, S* u) const {
         load_state<DIM, NS, S>(U, dU, c, u);
     }
-    __device__ __forceinline__ double temperature(int c) const { return __ldg(tmp + c); }
+    __device__ __forceinline__ double temperature(int c) const { return __ldg(tmp + (std::is_same<G, Dual>::value ? 2 * (size_t)c : (size_t)c)); }
     template <class S>
     __device__ __forceinline__ void aux_of(const Phys& P, const S* u, int c, S* a) const {
         cell_aux<DIM, NS>(P, u, tmp, c, a);
@@ -319,6 +319,21 @@ __global__ void __launch_bounds__(256) k_aux(DevMesh M, Phys P, const double* __
     for (int d = 0; d < DIM; d++) a[1 + d] = u[2 + d] * irho;
 ABL_UNROLL_SPECIES
     for (int s = 0; s < NS; s++) a[1 + DIM + s] = u[D::NE + s] * irho;
+    if (!ok) atomicOr(status, kStatusEos);
+}
+
+// (T, dT) of every cell for a tangent evaluation, from the temperatures that k_aux left: dT by the
+// implicit-function theorem, once per cell instead of once per neighbour and face
+template <int DIM, int NS>
+__global__ void __launch_bounds__(256) k_aux_tangent(DevMesh M, Phys P, const double* __restrict__ U, const double* __restrict__ dU,
+                                                     const double* __restrict__ tmp, double2* __restrict__ out, int* status) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= M.n_cells) return;
+    Dual u[Dims<DIM, NS>::NC];
+    load_state<DIM, NS, Dual>(U, dU, c, u);
+    bool ok = true;
+    const Dual T = temperature<DIM, NS>(P, NS, u, __ldg(tmp + c), &ok);
+    out[c] = make_double2(T.v, T.d);
     if (!ok) atomicOr(status, kStatusEos);
 }
 
@@ -397,6 +412,41 @@ ABL_UNROLL_SPECIES
     }
 }
 
+// The limiter of a tangent evaluation: the factor of a component is that of its minimising face, so the
+// values run through limit_field (which records that face) and the tangent is evaluated there alone, by the
+// dual-number form of the same expressions. On dual numbers throughout, the factors of all faces were two
+// thirds of the tangent gradient's instructions.
+template <int DIM, int NS, int LIM>
+__device__ __forceinline__ void limit_field_tangent(const DevMesh& M, const Phys& P, int beg, int end, size_t wb, const double* __restrict__ U,
+                                                    const double* __restrict__ dU, const Dual* uc, Dual* g, int k0, int k1, const double* sd) {
+    using D = Dims<DIM, NS>;
+    double gv[D::NC * DIM], ucv[D::NC], phi[D::NC];
+    int ist[D::NC];
+ABL_UNROLL_SPECIES
+    for (int k = 0; k < D::NC; k++) {
+        ucv[k] = uc[k].v;
+#pragma unroll
+        for (int d = 0; d < DIM; d++) gv[k * DIM + d] = g[k * DIM + d].v;
+    }
+    limit_field<DIM, NS, double, LIM, true>(M, P, beg, end, wb, U, nullptr, ucv, gv, k0, k1, phi, ist, sd);
+ABL_UNROLL_SPECIES
+    for (int k = 0; k < D::NC; k++) {
+        if (k < k0 || k >= k1) continue;
+        Dual f(phi[k]);
+        if (!P.jvp_frozen_limiter && ist[k] >= 0) {
+            const int i = ist[k];
+            const size_t e = (size_t)(M.cone[i].y & kConeNbr) * D::NC + k;
+            Dual denom = 0.0;
+#pragma unroll
+            for (int d = 0; d < DIM; d++) denom += g[k * DIM + d] * __ldg(M.cv + 3 * (wb + (size_t)(i - beg)) + d);
+            const Dual flim = 0.5 * (Dual(__ldg(U + e), __ldg(dU + e)) - uc[k]) * rcp64(denom);
+            f.d = limiter_k<LIM, Dual>(P.limiter, flim).d;
+        }
+#pragma unroll
+        for (int d = 0; d < DIM; d++) g[k * DIM + d] *= f;
+    }
+}
+
 // One thread per cell: one pass over the cell's faces accumulates the LSQ gradient of the conserved
 // fields (non-boundary faces, cgrad weights) and of the aux fields (all faces, fgrad weights), a second
 // pass applies the limiter. Cells without a conserved-state gradient (boundary ghosts, outer halo) get
@@ -429,8 +479,12 @@ ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NC * DIM; k++) g[k] = G(0);
 ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NA * DIM; k++) ga[k] = G(0);
+    // value and tangent of both gradients do not fit in the registers: a pass over the cone for each
+    constexpr bool kTwo = std::is_same<G, Dual>::value && NS > 0 && kUnrolled<NS>;
     // neighbour differences kept for the limiter when the block has shared memory for them
-    G* sd = (cache && state && P.limiter != ABL_LIMITER_NONE && end - beg <= M.max_cone) ? reinterpret_cast<G*>(gsm) : nullptr;
+    // (their values, in a tangent evaluation)
+    using C = typename std::conditional<std::is_same<G, Dual>::value && kUnrolled<NS>, double, G>::type;
+    C* sd = (cache && state && P.limiter != ABL_LIMITER_NONE && end - beg <= M.max_cone) ? reinterpret_cast<C*>(gsm) : nullptr;
     if (state || auxg) {
 #pragma unroll 1
         for (int i = beg; i < end; i++) {
@@ -440,7 +494,7 @@ ABL_UNROLL_SPECIES
             load_state<DIM, NS, S>(U, dU, n, un);
             if (sd) {
 ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NC; k++) sd[((i - beg) * D::NC + k) * blockDim.x + threadIdx.x] = G(un[k] - uc[k]);
+                for (int k = 0; k < D::NC; k++) sd[((i - beg) * D::NC + k) * blockDim.x + threadIdx.x] = C(un[k] - uc[k]);
             }
             G wd[DIM], wad[DIM];
             cone_weights<DIM, G>(M.cwa, M.cwa32, wb + (size_t)(i - beg), wd, wad);
@@ -452,7 +506,7 @@ ABL_UNROLL_SPECIES
                     for (int d = 0; d < DIM; d++) g[k * DIM + d] += wd[d] * delta;
                 }
             }
-            if (auxg) {
+            if (auxg && !kTwo) {
                 S an[D::NA];
                 cell_aux<DIM, NS>(P, un, tmp, n, an);
 ABL_UNROLL_SPECIES
@@ -484,12 +538,34 @@ ABL_UNROLL_SPECIES
                     rist[k * M.gs + c] = is[k];
                 }
             }
+        } else if constexpr (std::is_same<G, Dual>::value && kUnrolled<NS>) {
+            if (state && P.limiter != ABL_LIMITER_NONE) {
+                limit_field_tangent<DIM, NS, LIM>(M, P, beg, end, wb, U, dU, uc, g, 0, D::NE, sd);
+                if (NS > 0) limit_field_tangent<DIM, NS, LIM>(M, P, beg, end, wb, U, dU, uc, g, D::NE, D::NC, sd);
+            }
         } else if (state && P.limiter != ABL_LIMITER_NONE) {
             limit_field<DIM, NS, G, LIM>(M, P, beg, end, wb, U, dU, uc, g, 0, D::NE, nullptr, nullptr, sd);
             if (NS > 0) limit_field<DIM, NS, G, LIM>(M, P, beg, end, wb, U, dU, uc, g, D::NE, D::NC, nullptr, nullptr, sd);
         }
     }
     if (do_state) store_comps<GC::S>(grad, M.gs, c, g);
+    if (kTwo && auxg) {
+#pragma unroll 1
+        for (int i = beg; i < end; i++) {
+            const int n = M.cone[i].y & kConeNbr;
+            S un[D::NC], an[D::NA];
+            load_state<DIM, NS, S>(U, dU, n, un);
+            cell_aux<DIM, NS>(P, un, tmp, n, an);
+            G wd[DIM], wad[DIM];
+            cone_weights<DIM, G>(M.cwa, M.cwa32, wb + (size_t)(i - beg), wd, wad);
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NA; k++) {
+                const G delta = G(an[k] - ac[k]);
+#pragma unroll
+                for (int d = 0; d < DIM; d++) ga[k * DIM + d] += wad[d] * delta;
+            }
+        }
+    }
     if (do_aux) {
         G sa[GC::A];
         pack_aux_gradient<DIM, NS>(ga, sa);
@@ -838,9 +914,19 @@ __device__ __forceinline__ void face_geometry(const DevMesh& M, int i, double* n
 }
 
 // ---------------------------------------------------------------------------------------------------
+// what k_tile_flux keeps of a face flux: the flux, or a dual flux's tangent alone
+template <bool TAN, class S>
+__device__ __forceinline__ auto flux_part(S x) {
+    if constexpr (TAN)
+        return x.d;
+    else
+        return x;
+}
+
 // One CTA per tile. Phase 1: face fluxes into shared memory (tile-ordered geometry streamed from HBM).
 // Phase 2: each tile cell sums -+flux of its faces in ascending face order, adds the sum / V and writes F once.
-template <int DIM, int NS, class G, int FK>
+// TAN (a tangent without its value, the JVP's ordinary call): the records and the sums hold the tangent only.
+template <int DIM, int NS, class G, int FK, bool TAN = false>
 __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMesh M, Phys P, const double* __restrict__ U,
                                                                      const double* __restrict__ dU, const double* __restrict__ tmp,
                                                                      const G* __restrict__ grad, const G* __restrict__ agrad,
@@ -848,8 +934,9 @@ __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMe
                                                                      int* status, int t0 = 0) {
     using D = Dims<DIM, NS>;
     using S = StateOf<G>;
+    using T = typename std::conditional<TAN, double, S>::type;
     extern __shared__ double sflux_raw[];
-    S* sflux = reinterpret_cast<S*>(sflux_raw);  // [faces of this tile][NC]
+    T* sflux = reinterpret_cast<T*>(sflux_raw);  // [faces of this tile][NC]
     const int t = t0 + blockIdx.x;
     const int fb = M.tile_face_ptr[t], fe = M.tile_face_ptr[t + 1];
     bool ok = true, rok = true;
@@ -860,9 +947,9 @@ __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMe
         face_geometry<DIM, G>(M, i, normal, fdx);
         S flux[D::NC];
         face_flux<DIM, NS, G, FK>(P, src, lr.x, lr.y, normal, fdx, flux, &ok, &rok);
-        S* out = sflux + (size_t)(i - fb) * D::NC;
+        T* out = sflux + (size_t)(i - fb) * D::NC;
 ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) out[k] = flux[k];
+        for (int k = 0; k < D::NC; k++) out[k] = flux_part<TAN>(flux[k]);
     }
     __syncthreads();
     const int cb = M.tile_cell_ptr[t], ce = M.tile_cell_ptr[t + 1];
@@ -870,14 +957,16 @@ ABL_UNROLL_SPECIES
     for (int j = cb + threadIdx.x; j < ce; j += blockDim.x) {
         const int c = M.tile_cells[j];
         const double iv = M.ivol[c];
-        S acc[D::NC];
+        T acc[D::NC];
         if (overwrite) {
 ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NC; k++) acc[k] = 0.0;
         } else {
 ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NC; k++) {
-                if constexpr (std::is_same<S, Dual>::value)
+                if constexpr (TAN)
+                    acc[k] = dF[(size_t)c * D::NC + k];
+                else if constexpr (std::is_same<S, Dual>::value)
                     acc[k] = Dual(F ? F[(size_t)c * D::NC + k] : 0.0, dF[(size_t)c * D::NC + k]);
                 else
                     acc[k] = F[(size_t)c * D::NC + k];
@@ -886,13 +975,13 @@ ABL_UNROLL_SPECIES
         // the signed face fluxes summed first, then scaled by 1/V once: equal and opposite fluxes cancel
         // exactly (a uniform state keeps a zero residual, as the reference's per-face division gives;
         // a per-face fma(flux, 1/V, acc) would leave the rounding error of the product instead)
-        S sum[D::NC];
+        T sum[D::NC];
 ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NC; k++) sum[k] = 0.0;
         const int e0 = M.tc_fptr[j], e1 = M.tc_fptr[j + 1];
         for (int e = e0; e < e1; e++) {
             const uint16_t code = M.tc_face[e];
-            const S* ff = sflux + (size_t)(code & 0x7fff) * D::NC;
+            const T* ff = sflux + (size_t)(code & 0x7fff) * D::NC;
             if (code & 0x8000) {
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NC; k++) sum[k] += ff[k];
@@ -905,7 +994,9 @@ ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NC; k++) acc[k] += sum[k] * iv;
 ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NC; k++) {
-            if constexpr (std::is_same<S, Dual>::value) {
+            if constexpr (TAN) {
+                dF[(size_t)c * D::NC + k] = acc[k];
+            } else if constexpr (std::is_same<S, Dual>::value) {
                 if (F) F[(size_t)c * D::NC + k] = acc[k].v;
                 dF[(size_t)c * D::NC + k] = acc[k].d;
             } else {

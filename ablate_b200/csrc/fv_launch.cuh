@@ -5,15 +5,21 @@
 
 namespace abl {
 
-template <int DIM, int NS, class G, int FK>
+// the mixture's temperatures that the face and gradient passes of type G read
+template <class G>
+const double* face_temperatures(const abl_fv* fv) {
+    return std::is_same<G, Dual>::value ? fv->tmpD.p : fv->tmp.p;
+}
+
+template <int DIM, int NS, class G, int FK, bool TAN = false>
 void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, const G* agrad, double* F, double* dF, int overwrite,
                  cudaStream_t s) {
-    auto kern = k_tile_flux<DIM, NS, G, FK>;
-    const int smem = fv->tile_smem * (std::is_same<G, Dual>::value ? 2 : 1);
+    auto kern = k_tile_flux<DIM, NS, G, FK, TAN>;
+    const int smem = fv->tile_smem * (std::is_same<G, Dual>::value && !TAN ? 2 : 1);
     if (smem > 227 * 1024) throw AblError(ABL_ERR_UNSUPPORTED, "tile flux buffer exceeds shared memory for this species count");
     ABL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (!fv->pipe_active) {
-        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->tmp.p, grad, agrad, F, dF, overwrite, fv->status.p, 0);
+        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, 0);
         check_launch();
         return;
     }
@@ -22,7 +28,7 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
     const int nch = fv->chunk_tile.empty() ? 0 : (int)fv->chunk_tile.size() - 1;
     if (nch == 0) {
         ABL_CUDA(cudaStreamWaitEvent(s, fv->ev_in[0], 0));
-        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->tmp.p, grad, agrad, F, dF, overwrite, fv->status.p, 0);
+        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, 0);
         check_launch();
         return;
     }
@@ -30,7 +36,7 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
         const int ta = fv->chunk_tile[q], tb = fv->chunk_tile[q + 1];
         ABL_CUDA(cudaStreamWaitEvent(s, fv->ev_in[q], 0));
         if (tb > ta) {
-            kern<<<tb - ta, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->tmp.p, grad, agrad, F, dF, overwrite, fv->status.p, ta);
+            kern<<<tb - ta, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, ta);
             check_launch();
         }
         ABL_CUDA(cudaEventRecord(fv->ev_chunk[q], s));
@@ -83,7 +89,7 @@ void launch_fused(abl_fv* fv, const double* U, double* F, int overwrite, cudaStr
 // shared memory for the neighbour differences the limiter reuses (none when it would not fit)
 template <int DIM, int NS, class G>
 size_t gradient_smem(const abl_fv* fv) {
-    const size_t b = (size_t)128 * fv->mesh.max_cone * Dims<DIM, NS>::NC * sizeof(G);
+    const size_t b = (size_t)128 * fv->mesh.max_cone * Dims<DIM, NS>::NC * (std::is_same<G, Dual>::value && kUnrolled<NS> ? sizeof(double) : sizeof(G));
     return b <= 48 * 1024 ? b : 0;
 }
 
@@ -94,7 +100,7 @@ void launch_gradient(abl_fv* fv, const double* U, const double* dU, G* grad, G* 
     const abl::DevBuf<int>* list = fv->rhs_phase == 0 ? &fv->grad_early : fv->rhs_phase == 1 ? &fv->grad_late : nullptr;
     const int n = list ? (int)list->n : fv->mesh.n_cells;
     if (n == 0) return;
-    k_gradient<DIM, NS, G, LIM><<<blocks_for(n, 128), 128, smem, s>>>(fv->mesh, fv->phys, U, dU, fv->tmp.p, grad, agrad, fv->need_state_grad,
+    k_gradient<DIM, NS, G, LIM><<<blocks_for(n, 128), 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, fv->need_state_grad,
                                                                    fv->need_aux_grad, smem > 0, nullptr, nullptr, nullptr, list ? list->p : nullptr, n);
     check_launch();
 }
@@ -195,15 +201,29 @@ void run_jvp(abl_fv* fv, const double* U, const double* dU, double* F, double* d
         mark(fv, "k_aux", s);
         k_aux<DIM, NS><<<blocks_for(M.n_cells, 256), 256, 0, s>>>(M, fv->phys, U, fv->aux.p, fv->tmp.p, fv->status.p);
         check_launch();
+        k_aux_tangent<DIM, NS><<<blocks_for(M.n_cells, 256), 256, 0, s>>>(M, fv->phys, U, dU, fv->tmp.p, reinterpret_cast<double2*>(fv->tmpD.p), fv->status.p);
+        check_launch();
     }
     Dual* grad = reinterpret_cast<Dual*>(fv->gradD.p);
     Dual* agrad = reinterpret_cast<Dual*>(fv->agradD.p);
+    // limiter and flux calculator fixed at compile time where a specialised kernel exists, as in the RHS
+    constexpr bool spec = kSpecialized<NS>;
     if (fv->need_state_grad || fv->need_aux_grad) {
         mark(fv, "k_gradient_tangent", s);
-        launch_gradient<DIM, NS, Dual, -1>(fv, U, dU, grad, agrad, s);
+        if (spec && fv->phys.limiter == ABL_LIMITER_MINMOD)
+            launch_gradient<DIM, NS, Dual, spec ? ABL_LIMITER_MINMOD : -1>(fv, U, dU, grad, agrad, s);
+        else
+            launch_gradient<DIM, NS, Dual, -1>(fv, U, dU, grad, agrad, s);
     }
     mark(fv, "k_tile_flux_tangent", s);
-    if (M.n_tiles > 0) launch_tile<DIM, NS, Dual, -1>(fv, U, dU, grad, agrad, F, dF, 0, s);
+    if (M.n_tiles > 0) {
+        if (F)
+            launch_tile<DIM, NS, Dual, -1>(fv, U, dU, grad, agrad, F, dF, 0, s);
+        else if (spec && fv->phys.flux == ABL_FLUX_AUSMPUP)
+            launch_tile<DIM, NS, Dual, spec ? ABL_FLUX_AUSMPUP : -1, true>(fv, U, dU, grad, agrad, nullptr, dF, 0, s);
+        else
+            launch_tile<DIM, NS, Dual, -1, true>(fv, U, dU, grad, agrad, nullptr, dF, 0, s);
+    }
     mark(fv, "end", s);
 }
 
