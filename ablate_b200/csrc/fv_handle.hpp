@@ -129,7 +129,8 @@ struct abl_fv {
     abl::DevBuf<double> ghost_normal, rmin;
     abl::DevBuf<abl_bc> bc_table;
     abl::DevBuf<unsigned long long> dt_bits;
-    abl::DevBuf<double> step_U1, step_F;
+    abl::DevBuf<double> step_U1, step_U2, step_F;
+    abl::Stage stage;  // the stage that the RHS of the running step call takes (b = 0: none)
     // ghosts grouped by interior neighbour (adjoint of the fill), per-ghost value adjoints
     int n_gseg = 0;
     abl::DevBuf<int> gseg_ptr, gseg_nbr, gseg_ghost;

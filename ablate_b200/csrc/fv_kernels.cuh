@@ -914,6 +914,16 @@ __device__ __forceinline__ void face_geometry(const DevMesh& M, int i, double* n
 }
 
 // ---------------------------------------------------------------------------------------------------
+// A Runge-Kutta stage taken with the residual: Uout = a U0 + b (Us + dt F) on the owned rows, Us the state that
+// the residual is of. b = 0: no stage, the residual itself is written. dt is the double whose bits the CFL
+// reduction left in *dt_bits when that is not null; it is then added to *time, when that is not null.
+struct Stage {
+    double a = 0.0, b = 0.0, dt = 0.0;
+    const double* U0 = nullptr;
+    const unsigned long long* dt_bits = nullptr;
+    double* time = nullptr;
+};
+
 // what k_tile_flux keeps of a face flux: the flux, or a dual flux's tangent alone
 template <bool TAN, class S>
 __device__ __forceinline__ auto flux_part(S x) {
@@ -924,14 +934,15 @@ __device__ __forceinline__ auto flux_part(S x) {
 }
 
 // One CTA per tile. Phase 1: face fluxes into shared memory (tile-ordered geometry streamed from HBM).
-// Phase 2: each tile cell sums -+flux of its faces in ascending face order, adds the sum / V and writes F once.
+// Phase 2: each tile cell sums -+flux of its faces in ascending face order, adds the sum / V and writes F once,
+// or takes its Runge-Kutta stage and writes its new state to F (not the buffer of U: other tiles read that).
 // TAN (a tangent without its value, the JVP's ordinary call): the records and the sums hold the tangent only.
 template <int DIM, int NS, class G, int FK, bool TAN = false>
 __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMesh M, Phys P, const double* __restrict__ U,
                                                                      const double* __restrict__ dU, const double* __restrict__ tmp,
                                                                      const G* __restrict__ grad, const G* __restrict__ agrad,
                                                                      double* __restrict__ F, double* __restrict__ dF, int overwrite,
-                                                                     int* status, int t0 = 0) {
+                                                                     int* status, int t0 = 0, Stage st = Stage()) {
     using D = Dims<DIM, NS>;
     using S = StateOf<G>;
     using T = typename std::conditional<TAN, double, S>::type;
@@ -954,6 +965,8 @@ ABL_UNROLL_SPECIES
     __syncthreads();
     const int cb = M.tile_cell_ptr[t], ce = M.tile_cell_ptr[t + 1];
     bool finite = true;
+    const double dt = st.dt_bits ? __longlong_as_double((long long)*st.dt_bits) : st.dt;
+    if (st.time && t == 0 && threadIdx.x == 0) *st.time += dt;
     for (int j = cb + threadIdx.x; j < ce; j += blockDim.x) {
         const int c = M.tile_cells[j];
         const double iv = M.ivol[c];
@@ -992,6 +1005,18 @@ ABL_UNROLL_SPECIES
         }
 ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NC; k++) acc[k] += sum[k] * iv;
+        if constexpr (std::is_same<S, double>::value) {
+            if (st.b != 0.0) {
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NC; k++) {
+                    const size_t e = (size_t)c * D::NC + k;
+                    const double s = __ldg(U + e) + dt * acc[k];
+                    F[e] = st.a == 0.0 ? st.b * s : st.a * st.U0[e] + st.b * s;
+                    finite = finite && dfinite(acc[k]);
+                }
+                continue;
+            }
+        }
 ABL_UNROLL_SPECIES
         for (int k = 0; k < D::NC; k++) {
             if constexpr (TAN) {

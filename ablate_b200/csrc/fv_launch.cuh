@@ -19,7 +19,7 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
     if (smem > 227 * 1024) throw AblError(ABL_ERR_UNSUPPORTED, "tile flux buffer exceeds shared memory for this species count");
     ABL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (!fv->pipe_active) {
-        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, 0);
+        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, 0, fv->stage);
         check_launch();
         return;
     }
@@ -28,7 +28,7 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
     const int nch = fv->chunk_tile.empty() ? 0 : (int)fv->chunk_tile.size() - 1;
     if (nch == 0) {
         ABL_CUDA(cudaStreamWaitEvent(s, fv->ev_in[0], 0));
-        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, 0);
+        kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, 0, Stage());
         check_launch();
         return;
     }
@@ -36,7 +36,7 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
         const int ta = fv->chunk_tile[q], tb = fv->chunk_tile[q + 1];
         ABL_CUDA(cudaStreamWaitEvent(s, fv->ev_in[q], 0));
         if (tb > ta) {
-            kern<<<tb - ta, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, ta);
+            kern<<<tb - ta, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, ta, Stage());
             check_launch();
         }
         ABL_CUDA(cudaEventRecord(fv->ev_chunk[q], s));
