@@ -117,6 +117,7 @@ Phys make_phys(const abl_physics_desc* p) {
     P.k = p->k;
     P.mu = p->mu;
     P.diff = p->diff;
+    constant_terms(P);
     return P;
 }
 
@@ -1215,6 +1216,7 @@ int abl_flux_calculator_batch(int kind, double minf, double pgs_alpha, double ga
         P.minf = minf;
         P.alpha = pgs_alpha > 0 ? pgs_alpha : 1.0;
         P.gamma = gamma;
+        constant_terms(P);
         DevBuf<double> in, outd;
         DevBuf<int32_t> dir;
         DevBuf<int> st;

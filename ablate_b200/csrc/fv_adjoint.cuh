@@ -98,11 +98,10 @@ template <int DIM, int NSMAX>
 ABL_HD void decode_vjp(const Phys& P, int ns, const double* U, const Decoded<double>& dd, double eb, double ab, double pb, double* Ub) {
     const double rho = U[0];
     if (NSMAX == 0 || P.eos == ABL_EOS_PERFECT_GAS) {
-        const double cv = P.r_gas / (P.gamma - 1.0);
-        double Tb = eb * cv + pb * P.r_gas * rho;
+        double Tb = eb * P.cv + pb * P.r_gas * rho;
         if (dd.a > 0) Tb += ab * P.gamma * P.r_gas / (2.0 * dd.a);
         Ub[0] += pb * P.r_gas * dd.T;
-        internal_energy_vjp<DIM>(U, Tb * rcp64(cv), Ub);
+        internal_energy_vjp<DIM>(U, Tb * P.icv, Ub);
         return;
     }
     constexpr int NY = NSMAX > 0 ? NSMAX : 1;
@@ -214,7 +213,7 @@ ABL_UNROLL_SPECIES
         nasa_temperature_vjp<DIM, NS>(P, NS, u, ys, T, ab[0], ysb, Ub);
         fill_y_vjp<NS>(NS, u[0], u + D::NE, ysb, Ub, Ub + D::NE);
     } else {
-        internal_energy_vjp<DIM>(u, ab[0] * rcp64(P.r_gas / (P.gamma - 1.0)), Ub);
+        internal_energy_vjp<DIM>(u, ab[0] * P.icv, Ub);
     }
 }
 
@@ -323,14 +322,13 @@ struct AusmpupD {
     }
 };
 
-ABL_HD void ausmpup_vjp(double mInf, double alpha, const double* x, double mfb, double p12b, double* g) {
+ABL_HD void ausmpup_vjp(double mInf, double alpha, double ialpha, const double* x, double mfb, double p12b, double* g) {
     using A = Ausmpup<double>;
     using B = AusmpupD;
     const double uL = x[0], aL = x[1], rhoL = x[2], pL = x[3], uR = x[4], aR = x[5], rhoR = x[6], pR = x[7];
     const double Kp = 0.25, Ku = 0.75, sigma = 0.25;
     // forward
     const double rho12 = 0.5 * (rhoL + rhoR);
-    const double ialpha = rcp64(alpha);
     const double a12 = 0.5 * (aL + aR) * ialpha;
     const double ia12 = rcp64(a12);
     const double mL = uL * ia12, mR = uR * ia12;
@@ -353,7 +351,7 @@ ABL_HD void ausmpup_vjp(double mInf, double alpha, const double* x, double mfb, 
     const double p5P = A::P5P(mL, fa), p5M = A::P5M(mR, fa);
     // reverse
     double mLb = 0, mRb = 0, fab = 0, a12b = 0, rho12b = 0, mBar2b = 0;
-    const double vb = p12b * rcp64(sqr(alpha));
+    const double vb = p12b * sqr(ialpha);
     g[3] += vb * p5P;
     g[7] += vb * p5M;
     const double K = Ku * rho12 * fa * a12 * a12 * a2 * (mR - mL);
@@ -427,7 +425,7 @@ ABL_HD void calc_vjp(const Phys& P, const double* x, double mfb, double p12b, do
     if (kind == ABL_FLUX_AUSM)
         ausm_vjp(x, mfb, p12b, g);
     else if (kind == ABL_FLUX_AUSMPUP)
-        ausmpup_vjp(P.minf, P.alpha, x, mfb, p12b, g);
+        ausmpup_vjp(P.minf, P.alpha, P.ialpha, x, mfb, p12b, g);
     else
         calc_vjp_tangents(P, x, mfb, p12b, g, rok);
 }
@@ -454,13 +452,9 @@ __device__ __forceinline__ void advection_side_vjp(const Phys& P, const double* 
 // advection (NavierStokesTransport::AdvectionFlux + SpeciesTransport::AdvectionFlux) backwards: fb = flux
 // adjoint, ubL and ubR = adjoints of the two projected face states
 template <int DIM, int NS, int FK>
-__device__ __forceinline__ void advection_vjp(const Phys& P, const double* normal, const double* uL, const double* uR, double gsL, double gsR,
+__device__ __forceinline__ void advection_vjp(const Phys& P, const double* normal, double areaMag, const double* uL, const double* uR, double gsL, double gsR,
                                               bool adv, bool spadv, const double* fb, double* ubL, double* ubR, bool* ok, bool* rok) {
     using D = Dims<DIM, NS>;
-    double areaMag = 0;
-#pragma unroll
-    for (int d = 0; d < DIM; d++) areaMag += normal[d] * normal[d];
-    areaMag = sqrt(areaMag);
     const double iA = rcp64(areaMag);
     double norm[DIM];
 #pragma unroll
@@ -840,7 +834,7 @@ __global__ void __launch_bounds__(AdjBlocks<NS>::threads, AdjBlocks<NS>::tile) k
     if (dif || spdif) {
         for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
             const int2 lr = M.tf_cells[i];
-            double normal[DIM], fdx[6], flb[D::NC], fs[D::NC], fa[D::NA], gf[GC::A];
+            double normal[DIM], fdx[7], flb[D::NC], fs[D::NC], fa[D::NA], gf[GC::A];
             face_geometry<DIM, double>(M, i, normal, fdx);
             flux_adjoint<DIM, NS>(M, lr, Fb, flb);
             double wl = 0, wr = 0;
@@ -907,7 +901,7 @@ ABL_UNROLL_SPECIES
                 const uint16_t code = M.tc_face[e];
                 const int q = code & 0x7fff;
                 const double* r = srec + q;
-                double normal[DIM], fdx[6], gs[D::NA];
+                double normal[DIM], fdx[7], gs[D::NA];
                 face_geometry<DIM, double>(M, fb + q, normal, fdx);
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NA; k++) gs[k] = r[(AR::FG + k) * nf];
@@ -937,7 +931,7 @@ ABL_UNROLL_SPECIES
     if (adv || spadv) {
         for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
             const int2 lr = M.tf_cells[i];
-            double normal[DIM], fdx[6], uL[D::NC], uR[D::NC], flb[D::NC];
+            double normal[DIM], fdx[7], uL[D::NC], uR[D::NC], flb[D::NC];
             face_geometry<DIM, double>(M, i, normal, fdx);
             load_state<DIM, NS>(U, lr.x, uL);
             load_state<DIM, NS>(U, lr.y, uR);
@@ -965,7 +959,7 @@ ABL_UNROLL_SPECIES
             }
             flux_adjoint<DIM, NS>(M, lr, Fb, flb);
             double ubL[D::NC], ubR[D::NC];
-            advection_vjp<DIM, NS, FK>(P, normal, uL, uR, gsL, gsR, adv, spadv, flb, ubL, ubR, &ok, &rok);
+            advection_vjp<DIM, NS, FK>(P, normal, fdx[6], uL, uR, gsL, gsR, adv, spadv, flb, ubL, ubR, &ok, &rok);
             double* r = srec + (i - fb);
 ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NC; k++) {

@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         }
         for (int i = threadIdx.x; i < nf; i += blockDim.x) {
             const int lr = __ldg(faces + i);
-            double normal[DIM], fdx[6];
+            double normal[DIM], fdx[7];
             face_geometry_rec<DIM, G>(M, (size_t)__ldg(fgeo + i), normal, fdx);
             double flux[D::NC];
             face_flux<DIM, NS, G, FK>(P, src, lr & 0xffff, (int)((unsigned)lr >> 16), normal, fdx, flux, &ok, &rok);

@@ -44,7 +44,7 @@ struct DevMesh {
     const int* tile_cells;
     const int* tile_face_ptr;
     const int2* tf_cells;
-    const double* tf_geo;     // [ntf][10]: area normal (3), face centroid minus each side's centroid (6), pad
+    const double* tf_geo;     // [ntf][10]: area normal (3), face centroid minus each side's centroid (6), area
     const int* tc_fptr;
     const uint16_t* tc_face;
     // adjoint: records of faces with a non-owned side
@@ -243,7 +243,7 @@ __device__ __forceinline__ void aux_from_state(const Phys& P, const S* u, S* a) 
         a[1 + d] = u[2 + d] * irho;
         ke += a[1 + d] * a[1 + d];
     }
-    a[0] = (u[1] * irho - 0.5 * ke) * rcp64(P.r_gas / (P.gamma - 1.0));
+    a[0] = (u[1] * irho - 0.5 * ke) * P.icv;
 ABL_UNROLL_SPECIES
     for (int s = 0; s < NS; s++) a[1 + DIM + s] = u[D::NE + s] * irho;
 }
@@ -603,8 +603,7 @@ __device__ __forceinline__ void advection_split(const Phys& P, const double* nor
         unA[s] = un;
         const double eint = u[1] * irho[s] - 0.5 * v2;
         if (NS == 0 || P.eos == ABL_EOS_PERFECT_GAS) {
-            const double cv = P.r_gas / (P.gamma - 1.0);
-            const double T = eint * (1.0 / cv);
+            const double T = eint * P.icv;
             e[s] = eint;
             p[s] = P.r_gas * rho * T;
             a[s] = sqrtf(float(P.gamma * P.r_gas) * float(T));
@@ -708,10 +707,7 @@ ABL_UNROLL_SPECIES
         }
         if (!split) {
             // NavierStokesTransport::AdvectionFlux (navierStokesTransport.cpp:99-207)
-            double areaMag = 0;
-#pragma unroll
-            for (int d = 0; d < DIM; d++) areaMag += normal[d] * normal[d];
-            areaMag = sqrt(areaMag);
+            const double areaMag = fdx[6];
             const double iA = rcp64(areaMag);
             double norm[DIM];
 #pragma unroll
@@ -736,8 +732,7 @@ ABL_UNROLL_SPECIES
                     S v2 = 0;
 #pragma unroll
                     for (int d = 0; d < DIM; d++) v2 += velL[d] * velL[d];
-                    const S velMag = dsqrt(v2);
-                    const S H = dL.e + velMag * velMag / 2.0 + dL.p * irhoL;
+                    const S H = dL.e + 0.5 * v2 + dL.p * irhoL;
                     flux[1] = H * mf * areaMag;
 #pragma unroll
                     for (int n = 0; n < DIM; n++) flux[2 + n] = velL[n] * mf * areaMag + p12 * normal[n];
@@ -745,8 +740,7 @@ ABL_UNROLL_SPECIES
                     S v2 = 0;
 #pragma unroll
                     for (int d = 0; d < DIM; d++) v2 += velR[d] * velR[d];
-                    const S velMag = dsqrt(v2);
-                    const S H = dR.e + velMag * velMag / 2.0 + dR.p * irhoR;
+                    const S H = dR.e + 0.5 * v2 + dR.p * irhoR;
                     flux[1] = H * mf * areaMag;
 #pragma unroll
                     for (int n = 0; n < DIM; n++) flux[2 + n] = velR[n] * mf * areaMag + p12 * normal[n];
@@ -757,9 +751,8 @@ ABL_UNROLL_SPECIES
                         v2L += velL[d] * velL[d];
                         v2R += velR[d] * velR[d];
                     }
-                    const S mL = dsqrt(v2L), mR = dsqrt(v2R);
-                    const S HL = dL.e + mL * mL / 2.0 + dL.p * irhoL;
-                    const S HR = dR.e + mR * mR / 2.0 + dR.p * irhoR;
+                    const S HL = dL.e + 0.5 * v2L + dL.p * irhoL;
+                    const S HR = dR.e + 0.5 * v2R + dR.p * irhoR;
                     flux[1] = 0.5 * (HL + HR) * mf * areaMag;
 #pragma unroll
                     for (int n = 0; n < DIM; n++) flux[2 + n] = 0.5 * (velL[n] + velR[n]) * mf * areaMag + p12 * normal[n];
@@ -877,7 +870,7 @@ ABL_UNROLL_SPECIES
 }
 
 // ---------------------------------------------------------------------------------------------------
-// area normal and both sides' offsets of geometry record `rec` with vector loads
+// area normal, both sides' offsets fdx[0..5] and the area fdx[6] of geometry record `rec` with vector loads
 template <int DIM, class G>
 __device__ __forceinline__ void face_geometry_rec(const DevMesh& M, size_t rec, double* normal, double* fdx) {
     if constexpr (std::is_same<G, float>::value) {
@@ -893,6 +886,10 @@ __device__ __forceinline__ void face_geometry_rec(const DevMesh& M, size_t rec, 
             fdx[2 * q] = double(__int_as_float((int)(bits & 0xffffffffull)));
             fdx[2 * q + 1] = double(__int_as_float((int)(bits >> 32)));
         }
+        double a2 = 0;
+#pragma unroll
+        for (int d = 0; d < DIM; d++) a2 += normal[d] * normal[d];
+        fdx[6] = sqrt(a2);  // read by the calculators outside the AUSM family only
     } else {
         const double2* r = reinterpret_cast<const double2*>(M.tf_geo) + 5 * rec;
         const double2 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2), e = __ldg(r + 3), f = __ldg(r + 4);
@@ -905,6 +902,7 @@ __device__ __forceinline__ void face_geometry_rec(const DevMesh& M, size_t rec, 
         fdx[3] = e.x;
         fdx[4] = e.y;
         fdx[5] = f.x;
+        fdx[6] = f.y;
     }
 }
 // the same for tile face record i
@@ -954,7 +952,7 @@ __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMe
     const GlobalRows<DIM, NS, G> src{U, dU, tmp, grad, agrad, M.gs};
     for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
         const int2 lr = M.tf_cells[i];
-        double normal[DIM], fdx[6];
+        double normal[DIM], fdx[7];
         face_geometry<DIM, G>(M, i, normal, fdx);
         S flux[D::NC];
         face_flux<DIM, NS, G, FK>(P, src, lr.x, lr.y, normal, fdx, flux, &ok, &rok);

@@ -78,10 +78,18 @@ struct Phys {
     int32_t jvp_frozen_limiter;  // tangent evaluations hold the limiter factor at its value (dphi = 0)
     double gamma, r_gas, minf, alpha, max_lim_grad;
     double k, mu, diff;
+    double cv, icv, ialpha;  // r_gas / (gamma - 1) and its reciprocal (perfect gas), 1 / alpha: constant_terms
     const double* thermo; // [ns][14]: T_mid, a pad, then per range (low, high) the energy polynomial (species_poly)
     const double* inv_mw; // [ns]
     const double* diff_k; // [ns] per-species constant diffusivities (Constant model with one per species), or null
 };
+
+// what the kernels would divide for in every face
+inline void constant_terms(Phys& P) {
+    P.cv = P.r_gas / (P.gamma - 1.0);
+    P.icv = 1.0 / P.cv;
+    P.ialpha = 1.0 / P.alpha;
+}
 
 constexpr double kRuniv = 8314.46261815324;  // J/(kmol K)
 constexpr double kTref = 298.15;             // TChemBase::TREF (src/eos/tChemBase.hpp:150)
@@ -148,11 +156,11 @@ struct Ausmpup {
 };
 
 template <class R>
-ABL_HD int flux_ausmpup(R mInf, R pgsAlpha, R uL, R aL, R rhoL, R pL, R uR, R aR, R rhoR, R pR, R* mf, R* p12) {
+ABL_HD int flux_ausmpup(R mInf, R pgsAlpha, R ialpha, R uL, R aL, R rhoL, R pL, R uR, R aR, R rhoR, R pR, R* mf, R* p12) {
     using A = Ausmpup<R>;
     const R Kp = R(0.25), Ku = R(0.75), sigma = R(0.25);
     R rho12 = R(0.5) * (rhoL + rhoR);
-    R a12 = R(0.5) * (aL + aR) * rcp64(pgsAlpha);
+    R a12 = R(0.5) * (aL + aR) * ialpha;
     const R ia12 = rcp64(a12);
     R mL = uL * ia12;
     R mR = uR * ia12;
@@ -164,7 +172,7 @@ ABL_HD int flux_ausmpup(R mInf, R pgsAlpha, R uL, R aL, R rhoL, R pL, R uR, R aR
         R mO = dsqrt(mO2);
         fa = mO * (R(2) - mO);
     }
-    R m12 = A::M4P(mL) + A::M4M(mR) - (Kp * rcp64(fa)) * pmax(R(1) - (sigma * mBar2), R(0)) * (pR - pL) * rcp64(rho12 * a12 * a12 * pgsAlpha * pgsAlpha);
+    R m12 = A::M4P(mL) + A::M4M(mR) - Kp * pmax(R(1) - (sigma * mBar2), R(0)) * (pR - pL) * rcp64(fa * (rho12 * a12 * a12 * pgsAlpha * pgsAlpha));
     int dir;
     if (m12 > R(0)) {
         dir = ABL_DIR_LEFT;
@@ -177,7 +185,7 @@ ABL_HD int flux_ausmpup(R mInf, R pgsAlpha, R uL, R aL, R rhoL, R pL, R uR, R aR
         R p5Plus = A::P5P(mL, fa);
         R p5Minus = A::P5M(mR, fa);
         R v = p5Plus * pL + p5Minus * pR - Ku * p5Plus * p5Minus * rho12 * fa * a12 * a12 * pgsAlpha * pgsAlpha * (mR - mL);
-        *p12 = v * rcp64(sqr(pgsAlpha));
+        *p12 = v * sqr(ialpha);
     }
     return dir;
 }
@@ -312,7 +320,7 @@ ABL_HD int flux_calc(const Phys& P, R uL, R aL, R rhoL, R pL, R uR, R aR, R rhoR
         case ABL_FLUX_AUSM:
             return flux_ausm<R>(uL, aL, rhoL, pL, uR, aR, rhoR, pR, mf, p12);
         case ABL_FLUX_AUSMPUP:
-            return flux_ausmpup<R>(R(P.minf), R(P.alpha), uL, aL, rhoL, pL, uR, aR, rhoR, pR, mf, p12);
+            return flux_ausmpup<R>(R(P.minf), R(P.alpha), R(P.ialpha), uL, aL, rhoL, pL, uR, aR, rhoR, pR, mf, p12);
         case ABL_FLUX_RIEMANN:
             return flux_riemann<R>(R(P.gamma), uL, aL, rhoL, pL, uR, aR, rhoR, pR, mf, p12, ok);
         default:
@@ -325,7 +333,7 @@ ABL_HD int flux_calc(const Phys& P, R uL, R aL, R rhoL, R pL, R uR, R aR, R rhoR
 template <int FK, class R>
 ABL_HD int flux_calc_k(const Phys& P, R uL, R aL, R rhoL, R pL, R uR, R aR, R rhoR, R pR, R* mf, R* p12, bool* ok) {
     if constexpr (FK == ABL_FLUX_AUSM) return flux_ausm<R>(uL, aL, rhoL, pL, uR, aR, rhoR, pR, mf, p12);
-    if constexpr (FK == ABL_FLUX_AUSMPUP) return flux_ausmpup<R>(R(P.minf), R(P.alpha), uL, aL, rhoL, pL, uR, aR, rhoR, pR, mf, p12);
+    if constexpr (FK == ABL_FLUX_AUSMPUP) return flux_ausmpup<R>(R(P.minf), R(P.alpha), R(P.ialpha), uL, aL, rhoL, pL, uR, aR, rhoR, pR, mf, p12);
     return flux_calc<R>(P, uL, aL, rhoL, pL, uR, aR, rhoR, pR, mf, p12, ok);
 }
 
@@ -681,9 +689,8 @@ ABL_HD Decoded<S> decode(const Phys& P, int ns, const S* U, double Tguess, bool*
     if (NSMAX == 0 || P.eos == ABL_EOS_PERFECT_GAS) {
         // T = e/cv, e(T) = cv T, p(T) = R rho T, a(T) = sqrt(gamma p / rho) = sqrt(gamma R T)
         const S e = internal_energy<DIM>(U);
-        const double cv = P.r_gas / (P.gamma - 1.0);
-        d.T = e * rcp64(cv);
-        d.e = d.T * cv;
+        d.T = e * P.icv;
+        d.e = d.T * P.cv;
         d.p = P.r_gas * rho * d.T;
         d.a = dsqrt(P.gamma * P.r_gas * d.T);
         return d;
@@ -705,7 +712,7 @@ template <int DIM, int NSMAX, class S>
 ABL_HD S temperature(const Phys& P, int ns, const S* U, double Tguess, bool* ok) {
     if (NSMAX == 0 || P.eos == ABL_EOS_PERFECT_GAS) {
         const S e = internal_energy<DIM>(U);
-        return e * rcp64(P.r_gas / (P.gamma - 1.0));
+        return e * P.icv;
     }
     S ys[NSMAX > 0 ? NSMAX : 1];
     fill_y(ns, U[0], U + 2 + DIM, ys);

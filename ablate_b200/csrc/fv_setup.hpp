@@ -191,7 +191,7 @@ inline void lsq_pinv(int n, int dim, const double* B, double* W) {
 // the face geometry copied into tile order so the kernel streams it, and for every tile cell the
 // (local face, side) pairs in ascending global face order.
 //
-// The face records of a tile are in ascending face order. A face with a side that is not an owned cell (a
+// The face records of a tile are in ascending face order, axis by axis on an axis-aligned mesh. A face with a side that is not an owned cell (a
 // boundary ghost or a partition halo) is in exactly one tile; the adjoint's contribution to that side goes
 // to a per-face record (nb index).
 struct Tiles {
@@ -258,6 +258,21 @@ inline Tiles build_tiles(const HostMesh& h, const abl_mesh_desc* m, int tile_cel
     t.face_ptr.push_back(0);
     t.tc_fptr.assign(n + 1, 0);
     std::vector<std::vector<uint16_t>> lists;
+    std::vector<int> rec_of;
+    auto axis = [&](int f) {
+        const double* n = m->face_normal + 3 * (size_t)f;
+        int a = 0;
+        for (int d = 1; d < dim; d++)
+            if (std::fabs(n[d]) > std::fabs(n[a])) a = d;
+        return a;
+    };
+    bool aligned = true;
+    for (size_t q = 0; q < h.flux_faces.size() && aligned; q++) {
+        const double* n = m->face_normal + 3 * (size_t)h.flux_faces[q];
+        int nz = 0;
+        for (int d = 0; d < dim; d++) nz += n[d] != 0.0;
+        aligned = nz <= 1;
+    }
     t.face_nb.assign(h.n_faces, -1);
     for (int f : h.flux_faces)
         if (h.kind[h.face_cells[2 * f]] != ABL_CELL_OWNED || h.kind[h.face_cells[2 * f + 1]] != ABL_CELL_OWNED) t.face_nb[f] = t.n_nb++;
@@ -274,10 +289,15 @@ inline Tiles build_tiles(const HostMesh& h, const abl_mesh_desc* m, int tile_cel
         if (faces.size() > 0x7fff) throw std::invalid_argument("tile has too many faces");
         t.max_faces = std::max(t.max_faces, (int)faces.size());
         lists.assign(ce - cb, {});
-        // face records in global face order (the flux pass reads them in this order, neighbouring
-        // threads on neighbouring faces: the fastest of the orders measured)
+        // face records in global face order, on an axis-aligned mesh axis by axis: the lanes of a warp then hold
+        // faces of one direction, whose left and whose right cells are runs (128^3 box, face pass 456 -> 435 us)
+        rec_of.resize(faces.size());
+        std::vector<int> order(faces.size());
+        for (size_t i = 0; i < faces.size(); i++) order[i] = (int)i;
+        if (aligned) std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return axis(faces[a]) < axis(faces[b]); });
         for (size_t i = 0; i < faces.size(); i++) {
-            const int f = faces[i];
+            const int f = faces[order[i]];
+            rec_of[order[i]] = (int)i;
             const int L = h.face_cells[2 * f], R = h.face_cells[2 * f + 1];
             t.tf_cells.push_back(L);
             t.tf_cells.push_back(R);
@@ -290,8 +310,8 @@ inline Tiles build_tiles(const HostMesh& h, const abl_mesh_desc* m, int tile_cel
         for (size_t i = 0; i < faces.size(); i++) {
             const int f = faces[i];
             const int L = h.face_cells[2 * f], R = h.face_cells[2 * f + 1];
-            if (local[L] >= 0) lists[local[L]].push_back((uint16_t)i);
-            if (local[R] >= 0) lists[local[R]].push_back((uint16_t)(i | 0x8000));
+            if (local[L] >= 0) lists[local[L]].push_back((uint16_t)rec_of[i]);
+            if (local[R] >= 0) lists[local[R]].push_back((uint16_t)(rec_of[i] | 0x8000));
         }
         for (int j = cb; j < ce; j++) {
             t.tc_fptr[j + 1] = t.tc_fptr[j] + (int)lists[j - cb].size();
@@ -558,7 +578,7 @@ inline ConeRecords cone_records(const HostMesh& h, bool lsq, bool dif, bool tabl
 }
 
 // Per tile face record one 10-double geometry record: area normal (3), the face centroid minus each
-// side's centroid (6), a pad. With tables, records equal bit for bit are stored once and cls[i] gives
+// side's centroid (6), the area. With tables, records equal bit for bit are stored once and cls[i] gives
 // record i's copy.
 struct GeoRecords {
     std::vector<double> geo;
@@ -572,6 +592,8 @@ inline GeoRecords tile_geometry(const Tiles& tl, bool tables) {
     for (size_t i = 0; i < ntf; i++) {
         for (int d = 0; d < 3; d++) g.geo[10 * i + d] = tl.tf_normal[3 * i + d];
         for (int z = 0; z < 6; z++) g.geo[10 * i + 3 + z] = tl.tf_fdx[6 * i + z];
+        const double* n = &g.geo[10 * i];
+        g.geo[10 * i + 9] = std::sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
     }
     if (!tables || ntf < 8) return g;
     std::vector<int32_t> cls;
