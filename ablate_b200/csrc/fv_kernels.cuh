@@ -180,11 +180,12 @@ ABL_UNROLL_SPECIES
 // minimum resident CTAs per SM for __launch_bounds__ (register budget per thread = 65536 / (128 * n)),
 // chosen by timing: on the 128^3 gas gradient FP64 4 / FP32 6, tile FP64 4 (no spills at 128
 // registers) / FP32 5; with 3-5 species 3 (5 species: 2.7 % faster than 2), with more species 2 (9
-// species on tetrahedra: 3 is 14 % slower); the value+tangent pairs of the tangent kernels 3 without species
-// (168 registers; with one CTA's 250 the 64^3 channel's JVP took 342 us against 297) and 2 with
+// species on tetrahedra: 3 is 14 % slower); the value+tangent pairs of the tangent kernels: faces 3 without
+// species (168 registers; with one CTA's 250 the 64^3 channel's JVP took 342 us against 297), gradient 4 (128
+// registers in two passes over the cone; 3 with one pass: 96^3 box 399 us against 387), 2 with species
 template <int NS, class G>
 struct MinBlocks {
-    static constexpr int grad = std::is_same<G, Dual>::value ? (NS == 0 ? 3 : 2) : (NS > 5 ? 2 : (NS > 0 ? 3 : (sizeof(G) == 8 ? 4 : 6)));
+    static constexpr int grad = std::is_same<G, Dual>::value ? (NS == 0 ? 4 : 2) : (NS > 5 ? 2 : (NS > 0 ? 3 : (sizeof(G) == 8 ? 4 : 6)));
     static constexpr int tile = std::is_same<G, Dual>::value ? (NS == 0 ? 3 : 2) : (NS > 5 ? 2 : (NS > 2 ? 3 : (sizeof(G) == 8 ? 4 : 5)));
 };
 
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(256) k_aux_tangent(DevMesh M, Phys P, const do
 // cellInterpolant.cpp:282-328, and the cancel rule at :459-481)
 // REC (the adjoint's forward pass) also records, per component, the applied factor (0 when the
 // gradient was cancelled) and the cone entry of the minimising face (-1: none, or cancelled).
-// sd, when not null, holds the cell's neighbour differences u_n - u_c per cone entry (written by the
+// sd, when not null, holds half the cell's neighbour differences u_n - u_c per cone entry (written by the
 // gradient pass; thread-interleaved) so the neighbour states are not read again.
 template <int DIM, int NS, class G, int LIM, bool REC = false>
 __device__ __forceinline__ void limit_field(const DevMesh& M, const Phys& P, int beg, int end, size_t wb, const double* __restrict__ U,
@@ -371,16 +372,16 @@ ABL_UNROLL_SPECIES
             G denom = 0;
 #pragma unroll
             for (int d = 0; d < DIM; d++) denom += g[k * DIM + d] * v[d];
-            const G diff = sd ? sd[((i - beg) * D::NC + k) * blockDim.x + threadIdx.x] : G(un[k] - uc[k]);
-            const G flim = G(0.5) * diff * rcp64(denom);
+            const G half = sd ? sd[((i - beg) * D::NC + k) * blockDim.x + threadIdx.x] : G(0.5) * G(un[k] - uc[k]);
+            const G flim = half * rcp64(denom);
             if constexpr (REC) {
-                const G l = limiter_k<LIM, G>(P.limiter, flim);
+                const G l = limiter_key<LIM, G>(P.limiter, flim);
                 if (!(phi[k] < l)) {  // pmin(phi, l) takes l
                     phi[k] = l;
                     ist[k] = i;
                 }
             } else {
-                phi[k] = pmin(phi[k], limiter_k<LIM, G>(P.limiter, flim));
+                phi[k] = pmin(phi[k], limiter_key<LIM, G>(P.limiter, flim));
             }
         }
     }
@@ -389,6 +390,10 @@ ABL_UNROLL_SPECIES
 ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NC; k++) phi[k].d = 0.0;
         }
+    }
+    if constexpr (LIM == ABL_LIMITER_MINMOD) {
+ABL_UNROLL_SPECIES
+        for (int k = 0; k < D::NC; k++) phi[k] = limiter_value<LIM>(phi[k]);
     }
     bool cancel = false;
 ABL_UNROLL_SPECIES
@@ -480,7 +485,7 @@ ABL_UNROLL_SPECIES
 ABL_UNROLL_SPECIES
     for (int k = 0; k < D::NA * DIM; k++) ga[k] = G(0);
     // value and tangent of both gradients do not fit in the registers: a pass over the cone for each
-    constexpr bool kTwo = std::is_same<G, Dual>::value && NS > 0 && kUnrolled<NS>;
+    constexpr bool kTwo = std::is_same<G, Dual>::value && kUnrolled<NS>;
     // neighbour differences kept for the limiter when the block has shared memory for them
     // (their values, in a tangent evaluation)
     using C = typename std::conditional<std::is_same<G, Dual>::value && kUnrolled<NS>, double, G>::type;
@@ -494,7 +499,7 @@ ABL_UNROLL_SPECIES
             load_state<DIM, NS, S>(U, dU, n, un);
             if (sd) {
 ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NC; k++) sd[((i - beg) * D::NC + k) * blockDim.x + threadIdx.x] = C(un[k] - uc[k]);
+                for (int k = 0; k < D::NC; k++) sd[((i - beg) * D::NC + k) * blockDim.x + threadIdx.x] = C(0.5) * C(un[k] - uc[k]);
             }
             G wd[DIM], wad[DIM];
             cone_weights<DIM, G>(M.cwa, M.cwa32, wb + (size_t)(i - beg), wd, wad);

@@ -38,12 +38,12 @@ ABL_HD R sqr(R a) { return a * a; }
 // r <- r + r e by another (Markstein, "IA-64 and Elementary Functions", 2000, ch. 8): the first step
 // squares the relative error to about 2^-46, the second's residual is exact and leaves the result within
 // one ulp of 1/x (mostly the correctly rounded value). Zero, infinite, NaN and extreme inputs (|x|
-// outside 1e-300..1e300, where the approximation flushes subnormals) take the IEEE division, so their
-// special values are exactly those of 1/x.
+// outside 2^-996..2^996, where the approximation flushes subnormals) take the IEEE division, so their
+// special values are exactly those of 1/x; the range is checked on the exponent bits, off the FP64 pipe.
 ABL_HD double rcp64(double x) {
 #ifdef __CUDA_ARCH__
-    const double ax = fabs(x);
-    if (!(ax > 1e-300 && ax < 1e300)) return 1.0 / x;
+    const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    if (hi - 0x01b00000u >= 0x7e300000u - 0x01b00000u) return 1.0 / x;  // biased exponents 27 .. 2018
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     r = fma(r, fma(-x, r, 1.0), r);
@@ -789,6 +789,23 @@ ABL_HD R limiter(int kind, R f) {
         default:
             return R(1);
     }
+}
+
+// The factor in two parts, limiter_k = limiter_value(limiter_key): the key keeps the order of the factors, so
+// that the least factor over a cell's faces is that of the least key, and the rest runs once per cell.
+template <int LIM, class R>
+ABL_HD R limiter_key(int kind, R f) {
+    if constexpr (LIM == ABL_LIMITER_MINMOD)
+        return pmax(R(0), pmin(f, R(1) - f));
+    else
+        return limiter<R>(LIM >= 0 ? LIM : kind, f);
+}
+template <int LIM, class R>
+ABL_HD R limiter_value(R key) {
+    if constexpr (LIM == ABL_LIMITER_MINMOD)
+        return pmin(R(1), R(4) * key);
+    else
+        return key;
 }
 
 template <int LIM, class R>
