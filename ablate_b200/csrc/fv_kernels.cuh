@@ -490,10 +490,15 @@ ABL_UNROLL_SPECIES
     // (their values, in a tangent evaluation)
     using C = typename std::conditional<std::is_same<G, Dual>::value && kUnrolled<NS>, double, G>::type;
     C* sd = (cache && state && P.limiter != ABL_LIMITER_NONE && end - beg <= M.max_cone) ? reinterpret_cast<C*>(gsm) : nullptr;
+    // the next cone entry is loaded while this neighbour's row arrives (128^3 box 280 -> 269 us), where the
+    // registers hold it: with species or a tangent it spills (64^3 with five species 85 -> 90 us)
+    constexpr bool kAhead = NS == 0 && !std::is_same<G, Dual>::value;
     if (state || auxg) {
+        int2 next = kAhead && beg < end ? M.cone[beg] : make_int2(0, 0);
 #pragma unroll 1
         for (int i = beg; i < end; i++) {
-            const int2 ce = M.cone[i];
+            const int2 ce = kAhead ? next : M.cone[i];
+            if (kAhead && i + 1 < end) next = M.cone[i + 1];
             const int n = ce.y & kConeNbr;
             S un[D::NC];
             load_state<DIM, NS, S>(U, dU, n, un);
