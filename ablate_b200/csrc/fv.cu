@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(256) k_unpad_rows(const double* __restrict__ s
 const double* pad_in(abl_fv* fv, DevBuf<double>& scratch, const double* user, cudaStream_t s) {
     if (fv->pad == 0) return user;
     const size_t n = (size_t)fv->n_cells * fv->nc;
-    if (scratch.n != n) scratch.alloc(n);
+    scratch.ensure(n);
     k_pad_rows<<<blocks_for((long)n, 256), 256, 0, s>>>(user, fv->n_cells, fv->nc_user, 2 + fv->dim, fv->pad, scratch.p);
     check_launch();
     return scratch.p;
@@ -288,7 +288,7 @@ const double* pad_in(abl_fv* fv, DevBuf<double>& scratch, const double* user, cu
 // a zeroed residual buffer in the instance's width
 double* pad_out(abl_fv* fv, DevBuf<double>& scratch, cudaStream_t s) {
     const size_t n = (size_t)fv->n_cells * fv->nc;
-    if (scratch.n != n) scratch.alloc(n);
+    scratch.ensure(n);
     ABL_CUDA(cudaMemsetAsync(scratch.p, 0, n * sizeof(double), s));
     return scratch.p;
 }
@@ -963,9 +963,9 @@ int abl_fv_jvp(abl_fv* fv, double time, const double* U_dev, const double* dU_de
         if (!fv || !U_dev || !dU_dev || !dF_dev) throw std::invalid_argument("abl_fv_jvp: NULL argument");
         ABL_CUDA(cudaSetDevice(fv->device));
         // value + tangent gradient pairs, allocated on first use
-        if (fv->need_aux && fv->tmpD.n == 0) fv->tmpD.alloc((size_t)fv->n_cells * 2);
-        if (fv->need_state_grad && fv->gradD.n == 0) fv->gradD.alloc(fv->mesh.gs * fv->nc * fv->dim * 2);
-        if (fv->need_aux_grad && fv->agradD.n == 0) fv->agradD.alloc(fv->mesh.gs * aux_grad_comps(fv) * 2);
+        if (fv->need_aux) fv->tmpD.ensure((size_t)fv->n_cells * 2);
+        if (fv->need_state_grad) fv->gradD.ensure(fv->mesh.gs * fv->nc * fv->dim * 2);
+        if (fv->need_aux_grad) fv->agradD.ensure(fv->mesh.gs * aux_grad_comps(fv) * 2);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         if (fv->pad == 0) {
             dispatch_jvp(fv, U_dev, dU_dev, F_dev, dF_dev, s);
@@ -986,10 +986,10 @@ int abl_fv_jvp_host(abl_fv* fv, double time, const double* U_host, const double*
         if (!fv || !U_host || !dU_host || !dF_host) throw std::invalid_argument("abl_fv_jvp_host: NULL argument");
         ABL_CUDA(cudaSetDevice(fv->device));
         const size_t n = (size_t)fv->n_cells * fv->nc_user;
-        if (fv->hU.n != n) fv->hU.alloc(n);
-        if (fv->hdU.n != n) fv->hdU.alloc(n);
-        if (fv->hdF.n != n) fv->hdF.alloc(n);
-        if (F_host && fv->hF.n != n) fv->hF.alloc(n);
+        fv->hU.ensure(n);
+        fv->hdU.ensure(n);
+        fv->hdF.ensure(n);
+        if (F_host) fv->hF.ensure(n);
         ABL_CUDA(cudaMemcpy(fv->hU.p, U_host, n * sizeof(double), cudaMemcpyHostToDevice));
         ABL_CUDA(cudaMemcpy(fv->hdU.p, dU_host, n * sizeof(double), cudaMemcpyHostToDevice));
         ABL_CUDA(cudaMemcpy(fv->hdF.p, dF_host, n * sizeof(double), cudaMemcpyHostToDevice));
@@ -1007,22 +1007,19 @@ int abl_fv_vjp(abl_fv* fv, double time, const double* U_dev, const double* Fbar_
         if (!fv || !U_dev || !Fbar_dev || !Ubar_dev) throw std::invalid_argument("abl_fv_vjp: NULL argument");
         ABL_CUDA(cudaSetDevice(fv->device));
         // per-cell adjoint records, allocated on first use
-        const size_t n = (size_t)fv->n_cells;
-        if (fv->adj_ub.n == 0) {
-            const size_t gs = fv->mesh.gs;
-            if (fv->need_state_grad) fv->adj_gb.alloc(gs * fv->nc * fv->dim);
-            if (fv->need_aux_grad) fv->adj_gab.alloc(gs * aux_grad_comps(fv));
-            fv->adj_beta.alloc(gs * fv->nc);
-            fv->adj_fstar.alloc(gs * fv->nc);
-            fv->adj_ab.alloc(gs * fv->naux);
-            fv->adj_nb.alloc((size_t)std::max(fv->n_nb, 1) * (fv->nc + fv->nc * fv->dim + fv->naux + fv->naux * fv->dim));
-            fv->adj_ub.alloc(gs * fv->nc);
-            if (fv->need_state_grad) {
-                fv->adj_graw.alloc(gs * fv->nc * fv->dim);
-                fv->adj_phi.alloc(gs * fv->nc);
-                fv->adj_ist.alloc(gs * fv->nc);
-            }
+        const size_t gs = fv->mesh.gs;
+        if (fv->need_state_grad) {
+            fv->adj_gb.ensure(gs * fv->nc * fv->dim);
+            fv->adj_graw.ensure(gs * fv->nc * fv->dim);
+            fv->adj_phi.ensure(gs * fv->nc);
+            fv->adj_ist.ensure(gs * fv->nc);
         }
+        if (fv->need_aux_grad) fv->adj_gab.ensure(gs * aux_grad_comps(fv));
+        fv->adj_beta.ensure(gs * fv->nc);
+        fv->adj_fstar.ensure(gs * fv->nc);
+        fv->adj_ab.ensure(gs * fv->naux);
+        fv->adj_nb.ensure((size_t)std::max(fv->n_nb, 1) * (fv->nc + fv->nc * fv->dim + fv->naux + fv->naux * fv->dim));
+        fv->adj_ub.ensure(gs * fv->nc);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         if (fv->pad == 0) {
             dispatch_vjp(fv, U_dev, Fbar_dev, Ubar_dev, s);
@@ -1042,9 +1039,9 @@ int abl_fv_vjp_host(abl_fv* fv, double time, const double* U_host, const double*
         if (!fv || !U_host || !Fbar_host || !Ubar_host) throw std::invalid_argument("abl_fv_vjp_host: NULL argument");
         ABL_CUDA(cudaSetDevice(fv->device));
         const size_t n = (size_t)fv->n_cells * fv->nc_user;
-        if (fv->hU.n != n) fv->hU.alloc(n);
-        if (fv->hdU.n != n) fv->hdU.alloc(n);
-        if (fv->hdF.n != n) fv->hdF.alloc(n);
+        fv->hU.ensure(n);
+        fv->hdU.ensure(n);
+        fv->hdF.ensure(n);
         ABL_CUDA(cudaMemcpy(fv->hU.p, U_host, n * sizeof(double), cudaMemcpyHostToDevice));
         ABL_CUDA(cudaMemcpy(fv->hdF.p, Fbar_host, n * sizeof(double), cudaMemcpyHostToDevice));
         ABL_CUDA(cudaMemcpy(fv->hdU.p, Ubar_host, n * sizeof(double), cudaMemcpyHostToDevice));
@@ -1069,7 +1066,7 @@ int abl_fv_update_aux_host(abl_fv* fv, const double* U_host) {
         if (!fv || !U_host) throw std::invalid_argument("abl_fv_update_aux_host: NULL argument");
         ABL_CUDA(cudaSetDevice(fv->device));
         const size_t n = (size_t)fv->n_cells * fv->nc_user;
-        if (fv->hU.n != n) fv->hU.alloc(n);
+        fv->hU.ensure(n);
         ABL_CUDA(cudaMemcpy(fv->hU.p, U_host, n * sizeof(double), cudaMemcpyHostToDevice));
         int rc = abl_fv_update_aux(fv, fv->hU.p, nullptr);
         if (rc != ABL_OK) throw AblError(rc, g_last_error);
@@ -1086,8 +1083,8 @@ int abl_fv_rhs_host(abl_fv* fv, double time, const double* U_host, double* F_hos
         if (!fv || !U_host || !F_host) throw std::invalid_argument("abl_fv_rhs_host: NULL argument");
         ABL_CUDA(cudaSetDevice(fv->device));
         const size_t n = (size_t)fv->n_cells * fv->nc_user;
-        if (fv->hU.n != n) fv->hU.alloc(n);
-        if (fv->hF.n != n) fv->hF.alloc(n);
+        fv->hU.ensure(n);
+        fv->hF.ensure(n);
         if (fv->pad) {
             // a padded count: plain copies around the device call (no chunked overlap)
             ABL_CUDA(cudaMemcpy(fv->hU.p, U_host, n * sizeof(double), cudaMemcpyHostToDevice));
@@ -1333,8 +1330,13 @@ int abl_fv_set_boundary(abl_fv* fv, int32_t n_bc, const abl_bc* table, const int
                 if (gb[j] < 0 || gb[j] >= n_bc)
                     throw std::invalid_argument("abl_fv_set_boundary: boundary cell " + std::to_string(gc[j]) + " names no condition");
             }
-        fv->bc_table.upload(table, n_bc);
-        fv->ghost_bc.upload(gb.data(), gb.size());
+        // both are on the device before either replaces the handle's
+        DevBuf<abl_bc> tab;
+        DevBuf<int> idx;
+        tab.upload(table, n_bc);
+        idx.upload(gb.data(), gb.size());
+        fv->bc_table.swap(tab);
+        fv->ghost_bc.swap(idx);
         fv->n_bc = n_bc;
     });
 }
@@ -1361,7 +1363,7 @@ template <int DIM, int NS>
 void run_fill_ghosts_vjp(abl_fv* fv, double* Ub, cudaStream_t s) {
     if (fv->n_ghost == 0) return;
     const size_t n = (size_t)fv->n_ghost * fv->nc;
-    if (fv->ghost_vbar.n != n) fv->ghost_vbar.alloc(n);
+    fv->ghost_vbar.ensure(n);
     k_fill_ghosts_vjp<DIM, NS><<<blocks_for(fv->n_gseg, 256), 256, 0, s>>>(
         ghost_desc(fv), GhostSegments{fv->n_gseg, fv->gseg_ptr.p, fv->gseg_nbr.p, fv->gseg_ghost.p}, Ub, fv->ghost_vbar.p);
     check_launch();
@@ -1404,8 +1406,8 @@ void rk_stage_dev(abl_fv* fv, double a, const double* U0, double b, const double
 // fall away: ten steps of 256^2 cells, 826 -> 601 us with tiles of 128 cells.
 void ssprk3_staged(abl_fv* fv, double* U, int precision, double dt, const unsigned long long* dt_bits, double* time, cudaStream_t s) {
     const size_t n = (size_t)fv->n_cells * fv->nc;
-    if (fv->step_U1.n != n) fv->step_U1.alloc(n);
-    if (fv->step_U2.n != n) fv->step_U2.alloc(n);
+    fv->step_U1.ensure(n);
+    fv->step_U2.ensure(n);
     double *U1 = fv->step_U1.p, *U2 = fv->step_U2.p;
     if (fv->n_ghost + (int)fv->owned_rows.n != fv->n_cells) {
         // halo rows are neither owned nor filled from a condition: every buffer holds the caller's
@@ -1466,7 +1468,7 @@ int abl_fv_fill_ghosts_vjp(abl_fv* fv, double* Ubar_dev, double* value_bar_host,
         ABL_CUDA(cudaSetDevice(fv->device));
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const size_t nv = (size_t)fv->n_bc * ABL_BC_MAX_COMPONENTS;
-        if (fv->bc_vbar.n != nv) fv->bc_vbar.alloc(nv);
+        fv->bc_vbar.ensure(nv);
         ABL_CUDA(cudaMemsetAsync(fv->bc_vbar.p, 0, nv * sizeof(double), s));
         ABL_DISPATCH_EXACT(fv, run_fill_ghosts_vjp, Ubar_dev, s);
         if (value_bar_host) {
@@ -1489,11 +1491,12 @@ int abl_fv_set_pressure_functional(abl_fv* fv, int32_t n, const int32_t* cells, 
             if (seen[cells[j]]++) throw std::invalid_argument("abl_fv_set_pressure_functional: cell " + std::to_string(cells[j]) + " listed twice");
         }
         ABL_CUDA(cudaSetDevice(fv->device));
-        fv->fn_n = n;
+        fv->fn_n = 0;
         if (n == 0) return;
         fv->fn_cells.upload(cells, n);
         fv->fn_w.upload(weights, n);
         fv->fn_partial.alloc(blocks_for(n, 256));
+        fv->fn_n = n;
     });
 }
 
@@ -1561,7 +1564,7 @@ int abl_fv_step(abl_fv* fv, int scheme, double time, double dt, double* U_dev, i
         (void)time;
         ABL_DISPATCH_EXACT(fv, run_fill_ghosts, U_dev, s);
         const bool staged = scheme == ABL_STEP_SSPRK3 && stages_in_face_pass(fv);
-        if (!staged && fv->step_F.n != n) fv->step_F.alloc(n);
+        if (!staged) fv->step_F.ensure(n);
         double* F = fv->step_F.p;
         if (!staged) dispatch_rhs(fv, U_dev, F, precision, 1, s);
         if (staged) {
@@ -1570,7 +1573,7 @@ int abl_fv_step(abl_fv* fv, int scheme, double time, double dt, double* U_dev, i
             rk_stage(fv, 0.0, nullptr, 1.0, U_dev, dt, F, U_dev, s);
         } else {
             // U1 = U + dt L(U); U1 = 3/4 U + 1/4 (U1 + dt L(U1)); U = 1/3 U + 2/3 (U1 + dt L(U1))
-            if (fv->step_U1.n != n) fv->step_U1.alloc(n);
+            fv->step_U1.ensure(n);
             double* U1 = fv->step_U1.p;
             ABL_CUDA(cudaMemcpyAsync(U1, U_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
             rk_stage(fv, 0.0, nullptr, 1.0, U_dev, dt, F, U1, s);
@@ -1629,7 +1632,7 @@ int abl_fv_step_cfl(abl_fv* fv, int scheme, double cfl, double* U_dev, int preci
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const size_t n = (size_t)fv->n_cells * fv->nc;
         const bool staged = scheme == ABL_STEP_SSPRK3 && stages_in_face_pass(fv);
-        if (!staged && fv->step_F.n != n) fv->step_F.alloc(n);
+        if (!staged) fv->step_F.ensure(n);
         double* F = fv->step_F.p;
         // the CFL step of the state the step starts from, as abl_fv_cfl_dt computes it (ghosts filled first)
         ABL_DISPATCH_EXACT(fv, run_fill_ghosts, U_dev, s);
@@ -1640,7 +1643,7 @@ int abl_fv_step_cfl(abl_fv* fv, int scheme, double cfl, double* U_dev, int preci
         } else if (scheme == ABL_STEP_EULER) {
             rk_stage_dev(fv, 0.0, nullptr, 1.0, U_dev, F, U_dev, time_dev, s);
         } else {
-            if (fv->step_U1.n != n) fv->step_U1.alloc(n);
+            fv->step_U1.ensure(n);
             double* U1 = fv->step_U1.p;
             ABL_CUDA(cudaMemcpyAsync(U1, U_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
             rk_stage_dev(fv, 0.0, nullptr, 1.0, U_dev, F, U1, nullptr, s);

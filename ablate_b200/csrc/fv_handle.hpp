@@ -3,58 +3,16 @@
 #include <cuda_runtime.h>
 
 #include <cstdio>
-#include <stdexcept>
 #include <string>
 #include <vector>
 
 #include "fv_adjoint.cuh"
+#include "fv_devbuf.hpp"
 #include "fv_fused.cuh"
 
 namespace abl {
 
 extern thread_local std::string g_last_error;
-
-struct AblError : std::runtime_error {
-    int code;
-    AblError(int c, const std::string& m) : std::runtime_error(m), code(c) {}
-};
-
-#define ABL_CUDA(call)                                                                                           \
-    do {                                                                                                         \
-        cudaError_t e_ = (call);                                                                                 \
-        if (e_ != cudaSuccess) throw AblError(ABL_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
-    } while (0)
-
-template <class T>
-struct DevBuf {
-    T* p = nullptr;
-    size_t n = 0;
-    DevBuf() = default;
-    DevBuf(const DevBuf&) = delete;
-    DevBuf& operator=(const DevBuf&) = delete;
-    ~DevBuf() {
-        if (p) cudaFree(p);
-    }
-    void alloc(size_t count) {
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = count;
-        if (count == 0) return;
-        cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-        if (e != cudaSuccess) {
-            p = nullptr;
-            throw AblError(e == cudaErrorMemoryAllocation ? ABL_ERR_OUT_OF_MEMORY : ABL_ERR_CUDA,
-                           std::string("cudaMalloc: ") + cudaGetErrorString(e));
-        }
-    }
-    void upload(const T* h, size_t count) {
-        alloc(count);
-        if (count) ABL_CUDA(cudaMemcpy(p, h, count * sizeof(T), cudaMemcpyHostToDevice));
-    }
-    void zero() {
-        if (n) ABL_CUDA(cudaMemset(p, 0, n * sizeof(T)));
-    }
-};
 
 inline unsigned blocks_for(long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
