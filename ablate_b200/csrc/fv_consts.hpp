@@ -36,7 +36,8 @@ constexpr bool kSpecialized = NS <= 9;
 
 // Instances whose loops over the state components are unrolled (the others are the capacity instances,
 // ABL_CAPACITY_TU). Where a kernel has a second form, the capacity instances keep the first: their run-time
-// loops have returned wrong values from forms that are exact in every unrolled instance.
+// loops have returned wrong values from forms that are exact in every unrolled instance. In the 64-species
+// tangent that is the limiter on dual numbers and the face records with value and tangent, with F and without.
 template <int NS>
 constexpr bool kUnrolled = NS <= 16;
 
