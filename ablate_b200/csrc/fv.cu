@@ -571,8 +571,17 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
         fv->fdx.upload(h.fdx.data(), h.fdx.size());
         {
             std::vector<double> iv(h.n_cells);
-            for (int c = 0; c < h.n_cells; c++) iv[c] = 1.0 / mesh->cell_volume[c];
+            double ivmax = 0.0;
+            for (int c = 0; c < h.n_cells; c++) {
+                iv[c] = 1.0 / mesh->cell_volume[c];
+                if (h.kind[c] == ABL_CELL_OWNED) ivmax = std::max(ivmax, iv[c]);
+            }
             fv->ivol.upload(iv.data(), iv.size());
+            // a cell sums at most 2^15 faces (tc_face): fluxes below 2^(1008 - e), with every 1/V below 2^e, leave a
+            // residual below 2^1023. As the biased exponent; 0: no flux is known to be small enough
+            int e = 0;
+            std::frexp(ivmax, &e);
+            fv->mesh.flux_hi = std::isfinite(ivmax) ? (unsigned)std::max(0, 1023 + 1008 - std::max(e, 0)) << 20 : 0u;
         }
         // cell tiles for the fused flux kernel: the largest tile whose face fluxes fit in shared memory
         const int nc_ = 2 + h.dim + physics->n_species;

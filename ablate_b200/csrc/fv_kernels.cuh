@@ -30,6 +30,7 @@ struct DevMesh {
     int dim, n_cells, n_faces, n_flux_faces;
     const int2* face_cells;
     size_t gs;  // stride of one component of the per-cell gradient and adjoint arrays: n_cells, padded
+    unsigned flux_hi;  // face fluxes whose magnitudes' high words are below it sum to a finite residual in every cell
     const uint8_t* kind;
     const int* cone_ptr;
     // cone entry of a cell: x = face, y = neighbour | side << 31 | (face touches a boundary ghost) << 30
@@ -932,19 +933,15 @@ struct Stage {
     double* time = nullptr;
 };
 
-// what k_tile_flux keeps of a face flux: the flux, or a dual flux's tangent alone
-template <bool TAN, class S>
-__device__ __forceinline__ auto flux_part(S x) {
-    if constexpr (TAN)
-        return x.d;
-    else
-        return x;
-}
-
 // One CTA per tile. Phase 1: face fluxes into shared memory (tile-ordered geometry streamed from HBM).
 // Phase 2: each tile cell sums -+flux of its faces in ascending face order, adds the sum / V and writes F once,
 // or takes its Runge-Kutta stage and writes its new state to F (not the buffer of U: other tiles read that).
-// TAN (a tangent without its value, the JVP's ordinary call): the records and the sums hold the tangent only.
+// TAN (a tangent without its value, the JVP's ordinary call): the records and the sums hold the tangent only. A
+// residual that is not finite sets the status word all the same: where a face's value is so large that a sum of
+// them over V might not be finite (NaN and infinity among them; DevMesh::flux_hi, compared by the high word,
+// which orders magnitudes), the tile takes a second round, in which the records hold the values. That the values
+// are computed for the test costs 2 to 5 % of a JVP: 64^3 channel 244 -> 250 us, 60,000 tetrahedra with nine
+// species 402 -> 423 us.
 template <int DIM, int NS, class G, int FK, bool TAN = false>
 __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMesh M, Phys P, const double* __restrict__ U,
                                                                      const double* __restrict__ dU, const double* __restrict__ tmp,
@@ -958,85 +955,103 @@ __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMe
     T* sflux = reinterpret_cast<T*>(sflux_raw);  // [faces of this tile][NC]
     const int t = t0 + blockIdx.x;
     const int fb = M.tile_face_ptr[t], fe = M.tile_face_ptr[t + 1];
-    bool ok = true, rok = true;
+    bool ok = true, rok = true, finite = true;
     const GlobalRows<DIM, NS, G> src{U, dU, tmp, grad, agrad, M.gs};
-    for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
-        const int2 lr = M.tf_cells[i];
-        double normal[DIM], fdx[7];
-        face_geometry<DIM, G>(M, i, normal, fdx);
-        S flux[D::NC];
-        face_flux<DIM, NS, G, FK>(P, src, lr.x, lr.y, normal, fdx, flux, &ok, &rok);
-        T* out = sflux + (size_t)(i - fb) * D::NC;
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) out[k] = flux_part<TAN>(flux[k]);
-    }
-    __syncthreads();
-    const int cb = M.tile_cell_ptr[t], ce = M.tile_cell_ptr[t + 1];
-    bool finite = true;
-    const double dt = st.dt_bits ? __longlong_as_double((long long)*st.dt_bits) : st.dt;
-    if (st.time && t == 0 && threadIdx.x == 0) *st.time += dt;
-    for (int j = cb + threadIdx.x; j < ce; j += blockDim.x) {
-        const int c = M.tile_cells[j];
-        const double iv = M.ivol[c];
-        T acc[D::NC];
-        if (overwrite) {
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NC; k++) acc[k] = 0.0;
-        } else {
+    bool value = false;  // TAN: the round over the values
+#pragma unroll 1
+    for (;;) {
+        bool large = false;
+        for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
+            const int2 lr = M.tf_cells[i];
+            double normal[DIM], fdx[7];
+            face_geometry<DIM, G>(M, i, normal, fdx);
+            S flux[D::NC];
+            face_flux<DIM, NS, G, FK>(P, src, lr.x, lr.y, normal, fdx, flux, &ok, &rok);
+            T* out = sflux + (size_t)(i - fb) * D::NC;
 ABL_UNROLL_SPECIES
             for (int k = 0; k < D::NC; k++) {
-                if constexpr (TAN)
-                    acc[k] = dF[(size_t)c * D::NC + k];
-                else if constexpr (std::is_same<S, Dual>::value)
-                    acc[k] = Dual(F ? F[(size_t)c * D::NC + k] : 0.0, dF[(size_t)c * D::NC + k]);
-                else
-                    acc[k] = F[(size_t)c * D::NC + k];
+                if constexpr (TAN) {
+                    out[k] = value ? flux[k].v : flux[k].d;
+                    large |= ((unsigned)__double2hiint(flux[k].v) & 0x7fffffffu) >= M.flux_hi;
+                } else {
+                    out[k] = flux[k];
+                }
             }
         }
-        // the signed face fluxes summed first, then scaled by 1/V once: equal and opposite fluxes cancel
-        // exactly (a uniform state keeps a zero residual, as the reference's per-face division gives;
-        // a per-face fma(flux, 1/V, acc) would leave the rounding error of the product instead)
-        T sum[D::NC];
+        if constexpr (TAN)
+            large = __syncthreads_or(large);
+        else
+            __syncthreads();
+        const int cb = M.tile_cell_ptr[t], ce = M.tile_cell_ptr[t + 1];
+        const double dt = st.dt_bits ? __longlong_as_double((long long)*st.dt_bits) : st.dt;
+        if (st.time && t == 0 && threadIdx.x == 0) *st.time += dt;
+        for (int j = cb + threadIdx.x; j < ce; j += blockDim.x) {
+            const int c = M.tile_cells[j];
+            const double iv = M.ivol[c];
+            T acc[D::NC];
+            if (overwrite || (TAN && value)) {
 ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) sum[k] = 0.0;
-        const int e0 = M.tc_fptr[j], e1 = M.tc_fptr[j + 1];
-        for (int e = e0; e < e1; e++) {
-            const uint16_t code = M.tc_face[e];
-            const T* ff = sflux + (size_t)(code & 0x7fff) * D::NC;
-            if (code & 0x8000) {
-ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NC; k++) sum[k] += ff[k];
+                for (int k = 0; k < D::NC; k++) acc[k] = 0.0;
             } else {
-ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NC; k++) sum[k] -= ff[k];
-            }
-        }
-ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) acc[k] += sum[k] * iv;
-        if constexpr (std::is_same<S, double>::value) {
-            if (st.b != 0.0) {
 ABL_UNROLL_SPECIES
                 for (int k = 0; k < D::NC; k++) {
-                    const size_t e = (size_t)c * D::NC + k;
-                    const double s = __ldg(U + e) + dt * acc[k];
-                    F[e] = st.a == 0.0 ? st.b * s : st.a * st.U0[e] + st.b * s;
-                    finite = finite && dfinite(acc[k]);
+                    if constexpr (TAN)
+                        acc[k] = dF[(size_t)c * D::NC + k];
+                    else if constexpr (std::is_same<S, Dual>::value)
+                        acc[k] = Dual(F ? F[(size_t)c * D::NC + k] : 0.0, dF[(size_t)c * D::NC + k]);
+                    else
+                        acc[k] = F[(size_t)c * D::NC + k];
                 }
-                continue;
             }
-        }
+            // the signed face fluxes summed first, then scaled by 1/V once: equal and opposite fluxes cancel
+            // exactly (a uniform state keeps a zero residual, as the reference's per-face division gives;
+            // a per-face fma(flux, 1/V, acc) would leave the rounding error of the product instead)
+            T sum[D::NC];
 ABL_UNROLL_SPECIES
-        for (int k = 0; k < D::NC; k++) {
-            if constexpr (TAN) {
-                dF[(size_t)c * D::NC + k] = acc[k];
-            } else if constexpr (std::is_same<S, Dual>::value) {
-                if (F) F[(size_t)c * D::NC + k] = acc[k].v;
-                dF[(size_t)c * D::NC + k] = acc[k].d;
-            } else {
-                F[(size_t)c * D::NC + k] = acc[k];
+            for (int k = 0; k < D::NC; k++) sum[k] = 0.0;
+            const int e0 = M.tc_fptr[j], e1 = M.tc_fptr[j + 1];
+            for (int e = e0; e < e1; e++) {
+                const uint16_t code = M.tc_face[e];
+                const T* ff = sflux + (size_t)(code & 0x7fff) * D::NC;
+                if (code & 0x8000) {
+ABL_UNROLL_SPECIES
+                    for (int k = 0; k < D::NC; k++) sum[k] += ff[k];
+                } else {
+ABL_UNROLL_SPECIES
+                    for (int k = 0; k < D::NC; k++) sum[k] -= ff[k];
+                }
             }
-            finite = finite && dfinite(acc[k]);
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NC; k++) acc[k] += sum[k] * iv;
+            if constexpr (std::is_same<S, double>::value) {
+                if (st.b != 0.0) {
+ABL_UNROLL_SPECIES
+                    for (int k = 0; k < D::NC; k++) {
+                        const size_t e = (size_t)c * D::NC + k;
+                        const double s = __ldg(U + e) + dt * acc[k];
+                        F[e] = st.a == 0.0 ? st.b * s : st.a * st.U0[e] + st.b * s;
+                        finite = finite && dfinite(acc[k]);
+                    }
+                    continue;
+                }
+            }
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NC; k++) {
+                if constexpr (TAN) {
+                    if (!value) dF[(size_t)c * D::NC + k] = acc[k];
+                } else if constexpr (std::is_same<S, Dual>::value) {
+                    if (F) F[(size_t)c * D::NC + k] = acc[k].v;
+                    dF[(size_t)c * D::NC + k] = acc[k].d;
+                } else {
+                    F[(size_t)c * D::NC + k] = acc[k];
+                }
+                finite = finite && dfinite(acc[k]);
+            }
         }
+        if constexpr (!TAN) break;
+        if (value || !large) break;
+        value = true;
+        __syncthreads();  // the cells have read the records
     }
     if (!finite) atomicOr(status, kStatusNaN);
     if (!ok) atomicOr(status, kStatusEos);
