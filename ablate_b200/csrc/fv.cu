@@ -1428,8 +1428,8 @@ void ssprk3_staged(abl_fv* fv, double* U, int precision, double dt, const unsign
         ~Off() { fv->stage = Stage(); }
     } off{fv};
     auto stage = [&](double a, double b, const double* Us, double* Uout, double* t) {
-        fv->stage = Stage{a, b, dt, U, dt_bits, t};
-        dispatch_rhs(fv, Us, Uout, precision, 1, s);
+        fv->stage = Stage{a, b, dt, U, Uout, dt_bits, t};
+        dispatch_rhs(fv, Us, nullptr, precision, 1, s);
     };
     stage(0.0, 1.0, U, U1, nullptr);
     ABL_DISPATCH_EXACT(fv, run_fill_ghosts, U1, s);

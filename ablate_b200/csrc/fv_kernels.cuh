@@ -925,17 +925,20 @@ __device__ __forceinline__ void face_geometry(const DevMesh& M, int i, double* n
 // ---------------------------------------------------------------------------------------------------
 // A Runge-Kutta stage taken with the residual: Uout = a U0 + b (Us + dt F) on the owned rows, Us the state that
 // the residual is of. b = 0: no stage, the residual itself is written. dt is the double whose bits the CFL
-// reduction left in *dt_bits when that is not null; it is then added to *time, when that is not null.
+// reduction left in *dt_bits when that is not null; it is then added to *time, when that is not null. Uout may be
+// U0 (each thread reads its element before it writes it; neither pointer is __restrict__), not Us (other tiles
+// read that). U0 may be Us.
 struct Stage {
     double a = 0.0, b = 0.0, dt = 0.0;
     const double* U0 = nullptr;
+    double* Uout = nullptr;
     const unsigned long long* dt_bits = nullptr;
     double* time = nullptr;
 };
 
 // One CTA per tile. Phase 1: face fluxes into shared memory (tile-ordered geometry streamed from HBM).
 // Phase 2: each tile cell sums -+flux of its faces in ascending face order, adds the sum / V and writes F once,
-// or takes its Runge-Kutta stage and writes its new state to F (not the buffer of U: other tiles read that).
+// or takes its Runge-Kutta stage and writes its new state (F is not touched then).
 // TAN (a tangent without its value, the JVP's ordinary call): the records and the sums hold the tangent only. A
 // residual that is not finite sets the status word all the same: where a face's value is so large that a sum of
 // them over V might not be finite (NaN and infinity among them; DevMesh::flux_hi, compared by the high word,
@@ -1029,7 +1032,7 @@ ABL_UNROLL_SPECIES
                     for (int k = 0; k < D::NC; k++) {
                         const size_t e = (size_t)c * D::NC + k;
                         const double s = __ldg(U + e) + dt * acc[k];
-                        F[e] = st.a == 0.0 ? st.b * s : st.a * st.U0[e] + st.b * s;
+                        st.Uout[e] = st.a == 0.0 ? st.b * s : st.a * st.U0[e] + st.b * s;
                         finite = finite && dfinite(acc[k]);
                     }
                     continue;

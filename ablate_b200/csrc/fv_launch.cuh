@@ -23,6 +23,7 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
         check_launch();
         return;
     }
+    if (fv->stage.b != 0.0) throw AblError(ABL_ERR_UNSUPPORTED, "a host-buffer call takes no Runge-Kutta stage");
     // host-buffer call: each chunk of tiles waits for its residual rows, and once done sends them back on
     // the output stream while the next chunk runs
     const int nch = fv->chunk_tile.empty() ? 0 : (int)fv->chunk_tile.size() - 1;
