@@ -599,13 +599,8 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
             const size_t faces = (size_t)std::max(t.max_faces, 1) * nc_ * sizeof(double);
             return faces <= 200 * 1024 && 2 * faces <= 227 * 1024 && (size_t)std::max(t.max_faces, 1) * adj_row <= 227 * 1024;
         };
-        // 256 cells, or 128 with species: a tile's face records of either pass then leave room for the CTAs
-        // that the registers allow (five species, 256 cells: one CTA of the adjoint per SM instead of three)
-        int tile = physics->n_species > 0 && !fused_enabled() ? 128 : 256;
-        // and smaller on a mesh whose tiles would not fill the GPU, as long as all of them run at once (four
-        // CTAs per SM): such a mesh takes the time of one tile's chain of faces, not the sum of them
         const int64_t n_owned = std::count(h.kind.begin(), h.kind.end(), (uint8_t)ABL_CELL_OWNED);
-        while (tile > 32 && !fused_enabled() && n_owned <= (int64_t)(tile / 2) * 4 * fv->n_sm) tile /= 2;
+        int tile = fused_enabled() ? 256 : tile_cell_count(n_owned, physics->n_species, fv->n_sm);
         Tiles tl = tiles_for(tile);
         while (!fits(tl) && tile > 16) {
             tile /= 2;

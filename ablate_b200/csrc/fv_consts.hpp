@@ -34,6 +34,9 @@ constexpr int kMaxSpecies = 128;
 template <int NS>
 constexpr bool kSpecialized = NS <= 9;
 
+// CTAs per SM that the registers of the right-hand side's face pass let run at once (k_tile_flux in FP64)
+constexpr int face_pass_ctas(int ns) { return ns > 5 ? 2 : (ns > 2 ? 3 : 4); }
+
 // Instances whose loops over the state components are unrolled (the others are the capacity instances,
 // ABL_CAPACITY_TU). Where a kernel has a second form, the capacity instances keep the first: their run-time
 // loops have returned wrong values from forms that are exact in every unrolled instance. In the 64-species

@@ -187,7 +187,7 @@ ABL_UNROLL_SPECIES
 template <int NS, class G>
 struct MinBlocks {
     static constexpr int grad = std::is_same<G, Dual>::value ? (NS == 0 ? 4 : 2) : (NS > 5 ? 2 : (NS > 0 ? 3 : (sizeof(G) == 8 ? 4 : 6)));
-    static constexpr int tile = std::is_same<G, Dual>::value ? (NS == 0 ? 3 : 2) : (NS > 5 ? 2 : (NS > 2 ? 3 : (sizeof(G) == 8 ? 4 : 5)));
+    static constexpr int tile = std::is_same<G, Dual>::value ? (NS == 0 ? 3 : 2) : (NS > 2 || sizeof(G) == 8 ? face_pass_ctas(NS) : 5);
 };
 
 constexpr int kConeSide = int(1u << 31);

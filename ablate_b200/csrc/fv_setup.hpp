@@ -211,6 +211,25 @@ struct Tiles {
     int n_nb = 0;                         // number of such records
 };
 
+// Cells per tile of the face passes, before shared memory may ask for fewer. 256, or 128 with species: a tile's
+// face records of either pass then leave room for the CTAs that the registers allow (five species, 256 cells: one
+// CTA of the adjoint per SM instead of three). Fewer, down to 32, on a mesh whose tiles would not fill the GPU, as
+// long as all tiles of the right-hand side's face pass run at once: such a mesh takes the time of one tile's chain
+// of faces, not the sum of them. Right-hand side / JVP / VJP in us, of 32, 64 and 128 cells:
+//   gas, four CTAs per SM      27,000 cells  30 / 49 / 87    28 / 47 / 79    31 / 51 / 85
+//                              54,872        43 / 77 / 131   41 / 72 / 125   39 / 66 / 110
+//   five species, three        13,824        39 / 63 / 89    43 / 60 / 100   51 / 73 / 124
+//                              17,576        50 / 67 / 121   48 / 66 / 111   53 / 72 / 120
+//                              35,937        68 / 102 / 176  71 / 97 / 175   69 / 96 / 155
+//   nine species, two          13,824        52 / 90 / 143   51 / 88 / 122   61 / 110 / 148
+//     tetrahedra, about        30,000        97 / 226 / 364  96 / 227 / 310  85 / 195 / 243
+//     boxes                    35,937        84 / 164 / 264  80 / 161 / 229  79 / 154 / 271
+inline int tile_cell_count(int64_t n_owned, int n_species, int n_sm) {
+    int tile = n_species > 0 ? 128 : 256;
+    while (tile > 32 && n_owned <= (int64_t)(tile / 2) * face_pass_ctas(n_species) * n_sm) tile /= 2;
+    return tile;
+}
+
 inline uint64_t morton_spread(uint64_t x, int dim) {
     if (dim == 1) return x;
     uint64_t r = 0;

@@ -14,6 +14,9 @@ from oracle import oracle as orc
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(8, 4, 1), (11, 3, 1), (8, 8, 4), (43, 3, 2), (37, 32, 16), (61, 25, 13), (37, 32, 32), (53, 35, 21), (19, 73, 55)]
+# a wave of tiles on 148 SMs and a little more: three CTAs per SM with five species, two with nine
+SPECIES_SHAPES = [((37, 24, 16), 5), ((29, 35, 14), 5), ((37, 32, 24), 5), ((29, 28, 35), 5), ((37, 16, 16), 9), ((27, 27, 13), 9),
+                  ((37, 32, 16), 9), ((61, 25, 13), 9)]
 
 
 def _workload(shape, ns):
@@ -35,8 +38,7 @@ def _workload(shape, ns):
     return Workload("tiles", mesh, eos, procs, "leastsquares", "minmod", U, "tiles")
 
 
-@pytest.mark.parametrize("ns", [0, 5])
-@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shape,ns", [(shape, ns) for shape in SHAPES for ns in (0, 5)] + SPECIES_SHAPES)
 def test_passes_around_the_tile_limits(shape, ns):
     if ns and np.prod(shape) > 40000:
         pytest.skip("with species the tile size stops at 128 cells")
