@@ -2,7 +2,7 @@
 // ablate_b200/csrc/fv_physics.cuh) against the IEEE division 1/x computed on the host.
 //
 // Reads doubles from stdin-free generated inputs (the host builds them: log-uniform magnitudes over the
-// whole exponent range, both signs, the approximation's cut-offs 1e-300 and 1e300 with their neighbours,
+// whole exponent range, both signs, the approximation's cut-offs 2^-996 and 2^996 with their neighbours,
 // powers of two, mantissa extremes, zeros, subnormals, infinities and NaN), evaluates rcp64 on the
 // device, and prints one line: "n <count> max_ulp <worst error against the exact 1/x, in units of the last
 // place of the correctly rounded 1/x> not_nearest <results that are the neighbour of the correctly rounded
@@ -38,7 +38,7 @@ int main() {
         x.push_back((i & 1) ? -m : m);
     }
     for (int i = 0; i < 500000; i++) x.push_back(u01(rng) * ((i & 1) ? -1.0 : 1.0));  // dense mantissas in one binade
-    for (double t : {1e-300, 1e300}) {
+    for (double t : {0x1p-996, 0x1p996}) {
         double lo = t, hi = t;
         for (int k = 0; k < 64; k++) {
             x.push_back(lo);

@@ -1,7 +1,7 @@
 """Accuracy of the FP64 reciprocal the RHS kernels use for divisions that share a denominator.
 
 rcp64 (ablate_b200/csrc/fv_physics.cuh) refines the PTX rcp.approx.ftz.f64 approximation with two
-Newton-Raphson steps and sends zero, infinite, NaN and extreme inputs (|x| outside 1e-300..1e300) to the
+Newton-Raphson steps and sends zero, infinite, NaN and extreme inputs (|x| outside 2^-996..2^996) to the
 IEEE division. The check (tests/rcp64_check.cu, compiled here with nvcc for sm_100a) evaluates it on
 about 2.5 million inputs spanning the whole exponent range, the cut-offs and their neighbours, every
 power of two and the special values: the special values must equal the host's 1/x exactly, and every
