@@ -591,14 +591,9 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
             Tiles b = build_tiles(h, mesh, tile, true);
             return b.tf_cells.size() < a.tf_cells.size() ? b : a;
         };
-        // and whose shared memory fits every pass: the face fluxes (value and tangent pairs in the JVP) and
-        // the adjoint's face records (AdjRow::R)
-        const int naux_ = 1 + h.dim + physics->n_species;
-        const size_t adj_row = (size_t)std::max(naux_ + 2 + h.dim + physics->n_species, 2 * nc_) * sizeof(double);
-        auto fits = [&](const Tiles& t) {
-            const size_t faces = (size_t)std::max(t.max_faces, 1) * nc_ * sizeof(double);
-            return faces <= 200 * 1024 && 2 * faces <= 227 * 1024 && (size_t)std::max(t.max_faces, 1) * adj_row <= 227 * 1024;
-        };
+        // and whose shared memory fits every pass: two rows per face, of value and tangent in the JVP (with F) and
+        // of the two sides in the adjoint (AdjRow::R)
+        auto fits = [&](const Tiles& t) { return 2 * (size_t)std::max(t.max_faces, 1) * nc_ * sizeof(double) <= 227 * 1024; };
         const int64_t n_owned = std::count(h.kind.begin(), h.kind.end(), (uint8_t)ABL_CELL_OWNED);
         int tile = fused_enabled() ? 256 : tile_cell_count(n_owned, physics->n_species, fv->n_sm);
         Tiles tl = tiles_for(tile);
@@ -615,7 +610,7 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
         fv->tile_face_ptr.upload(tl.face_ptr.data(), tl.face_ptr.size());
         fv->tf_cells.upload(reinterpret_cast<const int2*>(tl.tf_cells.data()), tl.tf_cells.size() / 2);
         {
-            // per tile face one 80-byte record: normal, both offsets, a pad (five 16-byte loads), stored
+            // per tile face one 80-byte record: normal, both offsets, the area (five 16-byte loads), stored
             // once per distinct record where they repeat; the mixed path's 48-byte record holds the
             // normal and the offsets as FP32 pairs
             GeoRecords gr = tile_geometry(tl, record_tables());
@@ -1022,7 +1017,7 @@ int abl_fv_vjp(abl_fv* fv, double time, const double* U_dev, const double* Fbar_
         fv->adj_beta.ensure(gs * fv->nc);
         fv->adj_fstar.ensure(gs * fv->nc);
         fv->adj_ab.ensure(gs * fv->naux);
-        fv->adj_nb.ensure((size_t)std::max(fv->n_nb, 1) * (fv->nc + fv->nc * fv->dim + fv->naux + fv->naux * fv->dim));
+        fv->adj_nb.ensure((size_t)std::max(fv->n_nb, 1) * (fv->nc + fv->nc * fv->dim + fv->naux + aux_grad_comps(fv)));  // AdjRow::N
         fv->adj_ub.ensure(gs * fv->nc);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         if (fv->pad == 0) {

@@ -661,7 +661,8 @@ struct AdjRow {
     // shared-memory record of one face, [comp][face of the tile]: the diffusion pass leaves gs (NA), fab
     // (1+DIM) and fsb's density and species (1+NS; its others are 0), the advection pass ubL and ubR
     static constexpr int FG = 0, FA = D::NA, FS = D::NA + 1 + DIM;
-    static constexpr int R = FS + 1 + NS > 2 * D::NC ? FS + 1 + NS : 2 * D::NC;
+    static constexpr int R = 2 * D::NC;
+    static_assert(FS + 1 + NS <= R, "the advection pass's record is the larger");
 };
 
 // dF_L/dflux = -1/V_L, dF_R/dflux = +1/V_R on owned cells: the flux adjoint of a face
@@ -812,7 +813,7 @@ struct AdjBlocks {
 // such round each: a round's record is a third of both, and so are the live registers. Bound by the latency
 // of its loads and FP64 chains. Two lanes per face, both evaluating what couples the sides, with per-cell
 // accumulators in shared memory that the faces updated colour by colour, took 114 M warp instructions at
-// 64^3 cells; this takes 65 M, and a seventh of the shared-memory wavefronts.
+// 64^3 cells; this takes 60 M (523 -> 213 us).
 template <int DIM, int NS, int FK, int LIM>
 __global__ void __launch_bounds__(AdjBlocks<NS>::threads, AdjBlocks<NS>::tile) k_tile_adjoint(DevMesh M, Phys P, const double* __restrict__ U, const double* __restrict__ tmp,
                                                                           const double* __restrict__ grad, const double* __restrict__ agrad,

@@ -129,9 +129,9 @@ struct Dims {
 };
 
 // Components of the per-cell gradient arrays. They are stored component by component, [comp][cell]: the
-// face pass is bound by the L1's wavefronts (77 % of its peak with one row per cell, at 26 % of the issue
-// slots), and lanes on neighbouring cells then share a 128-byte line per component, where rows of 128 bytes
-// gave every lane a line of its own. The velocity part of the aux gradient is kept in the symmetric form that
+// face pass was bound by the L1's wavefronts with one row per cell (68 % of their peak at 26 % of the issue slots
+// on a 64^3 box; now 41 % at 36 %), and lanes on neighbouring cells then share a 128-byte line per component, where
+// rows of 128 bytes gave every lane a line of its own. The velocity part of the aux gradient is kept in the symmetric form that
 // the stress needs: du_c/dx_c, and du_c/dx_d + du_d/dx_c for c < d.
 template <int DIM, int NS>
 struct GradComps {
