@@ -543,7 +543,6 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
         fv->naux_user = fv->naux - pad;
         fv->n_cells = h.n_cells;
         fv->n_faces = h.n_faces;
-        fv->n_flux_faces = (int)h.flux_faces.size();
         fv->need_state_grad = lsq;
         fv->need_aux_grad = dif;
         // the mixture EOS keeps T resident (secant guess + face temperatures); a perfect gas recomputes it
@@ -554,7 +553,6 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
             fv->phys.diff_k = fv->diff_k.p;
         }
 
-        fv->face_cells.upload(reinterpret_cast<const int2*>(h.face_cells.data()), h.n_faces);
         fv->kind.upload(h.kind.data(), h.kind.size());
         fv->cone_ptr.upload(h.cone_ptr.data(), h.cone_ptr.size());
         {
@@ -662,8 +660,6 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
                 }
             }
         }
-        if (lsq) fv->cgrad.upload(h.cgrad.data(), h.cgrad.size());
-        if (dif) fv->fgrad.upload(h.fgrad.data(), h.fgrad.size());
         {
             // cone-major weights and offsets, one copy per distinct cell sequence where they repeat
             ConeRecords cr = cone_records(h, lsq, dif, record_tables());
@@ -810,18 +806,12 @@ int abl_fv_create(const abl_mesh_desc* mesh, const abl_physics_desc* physics, in
         }
 
         DevMesh& M = fv->mesh;
-        M.dim = fv->dim;
         M.n_cells = fv->n_cells;
-        M.n_faces = fv->n_faces;
-        M.n_flux_faces = fv->n_flux_faces;
-        M.face_cells = fv->face_cells.p;
         M.kind = fv->kind.p;
         M.cone_ptr = fv->cone_ptr.p;
         M.cone = fv->cone.p;
         M.fdx = fv->fdx.p;
         M.ivol = fv->ivol.p;
-        M.cgrad = fv->cgrad.p;
-        M.fgrad = fv->fgrad.p;
         M.n_tiles = tl.n_tiles;
         M.tile_cell_ptr = fv->tile_cell_ptr.p;
         M.tile_cells = fv->tile_cells.p;

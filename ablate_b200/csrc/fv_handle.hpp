@@ -32,14 +32,14 @@ struct abl_fv {
     // the caller's species in the instance's rows (0: the count has an instance of its own)
     int ns_user = 0, nc_user = 0, naux_user = 0, pad = 0;
     abl::DevBuf<double> pU, pdU, pF, pdF, pUb;  // rows in the instance's width when pad > 0
-    int n_cells = 0, n_faces = 0, n_flux_faces = 0;
+    int n_cells = 0, n_faces = 0;
     abl::Phys phys{};
     abl::DevMesh mesh{};
     // resident mesh + geometry
-    abl::DevBuf<int2> face_cells, cone;
+    abl::DevBuf<int2> cone;
     abl::DevBuf<uint8_t> kind;
     abl::DevBuf<int> cone_ptr;
-    abl::DevBuf<double> fdx, ivol, cgrad, fgrad;
+    abl::DevBuf<double> fdx, ivol;
     abl::DevBuf<double> thermo, diff_k;
     // tiles
     abl::DevBuf<int> tile_cell_ptr, tile_cells, tile_face_ptr, tc_fptr;

@@ -26,19 +26,17 @@ namespace abl {
 
 enum StatusBits : int { kStatusNaN = 1, kStatusEos = 2, kStatusRiemann = 4 };
 
+// passed by value with every launch: only what a kernel reads
 struct DevMesh {
-    int dim, n_cells, n_faces, n_flux_faces;
-    const int2* face_cells;
-    size_t gs;  // stride of one component of the per-cell gradient and adjoint arrays: n_cells, padded
+    int n_cells;
     unsigned flux_hi;  // face fluxes whose magnitudes' high words are below it sum to a finite residual in every cell
+    size_t gs;         // stride of one component of the per-cell gradient and adjoint arrays: n_cells, padded
     const uint8_t* kind;
     const int* cone_ptr;
     // cone entry of a cell: x = face, y = neighbour | side << 31 | (face touches a boundary ghost) << 30
     const int2* cone;
     const double* fdx;     // [nf][2][3] face centroid - side cell centroid (cell's own frame)
     const double* ivol;    // [nc] 1 / volume
-    const double* cgrad;   // [nf][2][3]
-    const double* fgrad;   // [nf][2][3]
     // tiles
     int n_tiles;
     const int* tile_cell_ptr;
