@@ -17,7 +17,8 @@ void launch_tile(abl_fv* fv, const double* U, const double* dU, const G* grad, c
     auto kern = k_tile_flux<DIM, NS, G, FK, TAN>;
     const int smem = fv->tile_smem * (std::is_same<G, Dual>::value && !TAN ? 2 : 1);
     if (smem > 227 * 1024) throw AblError(ABL_ERR_UNSUPPORTED, "tile flux buffer exceeds shared memory for this species count");
-    ABL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // up to 48 KB needs no opt-in, and a small call is bound by what the host does per launch
+    if (smem > 48 * 1024) ABL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (!fv->pipe_active) {
         kern<<<fv->mesh.n_tiles, 128, smem, s>>>(fv->mesh, fv->phys, U, dU, face_temperatures<G>(fv), grad, agrad, F, dF, overwrite, fv->status.p, 0, fv->stage);
         check_launch();
