@@ -941,8 +941,9 @@ struct Stage {
 // residual that is not finite sets the status word all the same: where a face's value is so large that a sum of
 // them over V might not be finite (NaN and infinity among them; DevMesh::flux_hi, compared by the high word,
 // which orders magnitudes), the tile takes a second round, in which the records hold the values. That the values
-// are computed for the test costs 2 to 5 % of a JVP: 64^3 channel 244 -> 250 us, 60,000 tetrahedra with nine
-// species 402 -> 423 us.
+// are computed for the test costs 2 to 3 % of a JVP, 9 % where the registers spill (64^3 channel 245 -> 250 us, 56^3
+// with five species 373 -> 378, 60,000 tetrahedra with nine 396 -> 434); the second round as a loop around the
+// first, with one copy of the flux, 2 to 8 % (252, 386, 433).
 template <int DIM, int NS, class G, int FK, bool TAN = false>
 __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMesh M, Phys P, const double* __restrict__ U,
                                                                      const double* __restrict__ dU, const double* __restrict__ tmp,
@@ -956,103 +957,120 @@ __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMe
     T* sflux = reinterpret_cast<T*>(sflux_raw);  // [faces of this tile][NC]
     const int t = t0 + blockIdx.x;
     const int fb = M.tile_face_ptr[t], fe = M.tile_face_ptr[t + 1];
-    bool ok = true, rok = true, finite = true;
+    bool ok = true, rok = true, large = false;
     const GlobalRows<DIM, NS, G> src{U, dU, tmp, grad, agrad, M.gs};
-    bool value = false;  // TAN: the round over the values
-#pragma unroll 1
-    for (;;) {
-        bool large = false;
-        for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
-            const int2 lr = M.tf_cells[i];
-            double normal[DIM], fdx[7];
-            face_geometry<DIM, G>(M, i, normal, fdx);
-            S flux[D::NC];
-            face_flux<DIM, NS, G, FK>(P, src, lr.x, lr.y, normal, fdx, flux, &ok, &rok);
-            T* out = sflux + (size_t)(i - fb) * D::NC;
+    for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
+        const int2 lr = M.tf_cells[i];
+        double normal[DIM], fdx[7];
+        face_geometry<DIM, G>(M, i, normal, fdx);
+        S flux[D::NC];
+        face_flux<DIM, NS, G, FK>(P, src, lr.x, lr.y, normal, fdx, flux, &ok, &rok);
+        T* out = sflux + (size_t)(i - fb) * D::NC;
 ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NC; k++) {
-                if constexpr (TAN) {
-                    out[k] = value ? flux[k].v : flux[k].d;
-                    large |= ((unsigned)__double2hiint(flux[k].v) & 0x7fffffffu) >= M.flux_hi;
-                } else {
-                    out[k] = flux[k];
-                }
+        for (int k = 0; k < D::NC; k++) {
+            if constexpr (TAN) {
+                out[k] = flux[k].d;
+                large |= ((unsigned)__double2hiint(flux[k].v) & 0x7fffffffu) >= M.flux_hi;
+            } else {
+                out[k] = flux[k];
             }
         }
-        if constexpr (TAN)
-            large = __syncthreads_or(large);
-        else
-            __syncthreads();
-        const int cb = M.tile_cell_ptr[t], ce = M.tile_cell_ptr[t + 1];
-        const double dt = st.dt_bits ? __longlong_as_double((long long)*st.dt_bits) : st.dt;
-        if (st.time && t == 0 && threadIdx.x == 0) *st.time += dt;
-        for (int j = cb + threadIdx.x; j < ce; j += blockDim.x) {
-            const int c = M.tile_cells[j];
-            const double iv = M.ivol[c];
-            T acc[D::NC];
-            if (overwrite || (TAN && value)) {
+    }
+    if constexpr (TAN)
+        large = __syncthreads_or(large);
+    else
+        __syncthreads();
+    const int cb = M.tile_cell_ptr[t], ce = M.tile_cell_ptr[t + 1];
+    bool finite = true;
+    const double dt = st.dt_bits ? __longlong_as_double((long long)*st.dt_bits) : st.dt;
+    if (st.time && t == 0 && threadIdx.x == 0) *st.time += dt;
+    for (int j = cb + threadIdx.x; j < ce; j += blockDim.x) {
+        const int c = M.tile_cells[j];
+        const double iv = M.ivol[c];
+        T acc[D::NC];
+        if (overwrite) {
 ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NC; k++) acc[k] = 0.0;
+            for (int k = 0; k < D::NC; k++) acc[k] = 0.0;
+        } else {
+ABL_UNROLL_SPECIES
+            for (int k = 0; k < D::NC; k++) {
+                if constexpr (TAN)
+                    acc[k] = dF[(size_t)c * D::NC + k];
+                else if constexpr (std::is_same<S, Dual>::value)
+                    acc[k] = Dual(F ? F[(size_t)c * D::NC + k] : 0.0, dF[(size_t)c * D::NC + k]);
+                else
+                    acc[k] = F[(size_t)c * D::NC + k];
+            }
+        }
+        // the signed face fluxes summed first, then scaled by 1/V once: equal and opposite fluxes cancel
+        // exactly (a uniform state keeps a zero residual, as the reference's per-face division gives;
+        // a per-face fma(flux, 1/V, acc) would leave the rounding error of the product instead)
+        T sum[D::NC];
+ABL_UNROLL_SPECIES
+        for (int k = 0; k < D::NC; k++) sum[k] = 0.0;
+        const int e0 = M.tc_fptr[j], e1 = M.tc_fptr[j + 1];
+        for (int e = e0; e < e1; e++) {
+            const uint16_t code = M.tc_face[e];
+            const T* ff = sflux + (size_t)(code & 0x7fff) * D::NC;
+            if (code & 0x8000) {
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NC; k++) sum[k] += ff[k];
             } else {
 ABL_UNROLL_SPECIES
-                for (int k = 0; k < D::NC; k++) {
-                    if constexpr (TAN)
-                        acc[k] = dF[(size_t)c * D::NC + k];
-                    else if constexpr (std::is_same<S, Dual>::value)
-                        acc[k] = Dual(F ? F[(size_t)c * D::NC + k] : 0.0, dF[(size_t)c * D::NC + k]);
-                    else
-                        acc[k] = F[(size_t)c * D::NC + k];
-                }
-            }
-            // the signed face fluxes summed first, then scaled by 1/V once: equal and opposite fluxes cancel
-            // exactly (a uniform state keeps a zero residual, as the reference's per-face division gives;
-            // a per-face fma(flux, 1/V, acc) would leave the rounding error of the product instead)
-            T sum[D::NC];
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NC; k++) sum[k] = 0.0;
-            const int e0 = M.tc_fptr[j], e1 = M.tc_fptr[j + 1];
-            for (int e = e0; e < e1; e++) {
-                const uint16_t code = M.tc_face[e];
-                const T* ff = sflux + (size_t)(code & 0x7fff) * D::NC;
-                if (code & 0x8000) {
-ABL_UNROLL_SPECIES
-                    for (int k = 0; k < D::NC; k++) sum[k] += ff[k];
-                } else {
-ABL_UNROLL_SPECIES
-                    for (int k = 0; k < D::NC; k++) sum[k] -= ff[k];
-                }
-            }
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NC; k++) acc[k] += sum[k] * iv;
-            if constexpr (std::is_same<S, double>::value) {
-                if (st.b != 0.0) {
-ABL_UNROLL_SPECIES
-                    for (int k = 0; k < D::NC; k++) {
-                        const size_t e = (size_t)c * D::NC + k;
-                        const double s = __ldg(U + e) + dt * acc[k];
-                        st.Uout[e] = st.a == 0.0 ? st.b * s : st.a * st.U0[e] + st.b * s;
-                        finite = finite && dfinite(acc[k]);
-                    }
-                    continue;
-                }
-            }
-ABL_UNROLL_SPECIES
-            for (int k = 0; k < D::NC; k++) {
-                if constexpr (TAN) {
-                    if (!value) dF[(size_t)c * D::NC + k] = acc[k];
-                } else if constexpr (std::is_same<S, Dual>::value) {
-                    if (F) F[(size_t)c * D::NC + k] = acc[k].v;
-                    dF[(size_t)c * D::NC + k] = acc[k].d;
-                } else {
-                    F[(size_t)c * D::NC + k] = acc[k];
-                }
-                finite = finite && dfinite(acc[k]);
+                for (int k = 0; k < D::NC; k++) sum[k] -= ff[k];
             }
         }
-        if constexpr (!TAN) break;
-        if (value || !large) break;
-        value = true;
-        __syncthreads();  // the cells have read the records
+ABL_UNROLL_SPECIES
+        for (int k = 0; k < D::NC; k++) acc[k] += sum[k] * iv;
+        if constexpr (std::is_same<S, double>::value) {
+            if (st.b != 0.0) {
+ABL_UNROLL_SPECIES
+                for (int k = 0; k < D::NC; k++) {
+                    const size_t e = (size_t)c * D::NC + k;
+                    const double s = __ldg(U + e) + dt * acc[k];
+                    st.Uout[e] = st.a == 0.0 ? st.b * s : st.a * st.U0[e] + st.b * s;
+                    finite = finite && dfinite(acc[k]);
+                }
+                continue;
+            }
+        }
+ABL_UNROLL_SPECIES
+        for (int k = 0; k < D::NC; k++) {
+            if constexpr (TAN) {
+                dF[(size_t)c * D::NC + k] = acc[k];
+            } else if constexpr (std::is_same<S, Dual>::value) {
+                if (F) F[(size_t)c * D::NC + k] = acc[k].v;
+                dF[(size_t)c * D::NC + k] = acc[k].d;
+            } else {
+                F[(size_t)c * D::NC + k] = acc[k];
+            }
+            finite = finite && dfinite(acc[k]);
+        }
+    }
+    if constexpr (TAN) {
+        if (large) {
+            __syncthreads();  // the cells have read the tangents
+#pragma unroll 1
+            for (int i = fb + threadIdx.x; i < fe; i += blockDim.x) {
+                const int2 lr = M.tf_cells[i];
+                double normal[DIM], fdx[7];
+                face_geometry<DIM, G>(M, i, normal, fdx);
+                S flux[D::NC];
+                face_flux<DIM, NS, G, FK>(P, src, lr.x, lr.y, normal, fdx, flux, &ok, &rok);
+                for (int k = 0; k < D::NC; k++) sflux[(size_t)(i - fb) * D::NC + k] = flux[k].v;
+            }
+            __syncthreads();
+            for (int j = cb + threadIdx.x; j < ce; j += blockDim.x)
+                for (int k = 0; k < D::NC; k++) {
+                    double sum = 0.0;
+                    for (int e = M.tc_fptr[j]; e < M.tc_fptr[j + 1]; e++) {
+                        const uint16_t code = M.tc_face[e];
+                        const double f = sflux[(size_t)(code & 0x7fff) * D::NC + k];
+                        sum += (code & 0x8000) ? f : -f;
+                    }
+                    finite = finite && dfinite(sum * M.ivol[M.tile_cells[j]]);
+                }
+        }
     }
     if (!finite) atomicOr(status, kStatusNaN);
     if (!ok) atomicOr(status, kStatusEos);
