@@ -941,9 +941,9 @@ struct Stage {
 // residual that is not finite sets the status word all the same: where a face's value is so large that a sum of
 // them over V might not be finite (NaN and infinity among them; DevMesh::flux_hi, compared by the high word,
 // which orders magnitudes), the tile takes a second round, in which the records hold the values. That the values
-// are computed for the test costs 2 to 3 % of a JVP, 9 % where the registers spill (64^3 channel 245 -> 250 us, 56^3
-// with five species 373 -> 378, 60,000 tetrahedra with nine 396 -> 434); the second round as a loop around the
-// first, with one copy of the flux, 2 to 8 % (252, 386, 433).
+// are computed for the test costs 2 to 3 % of a JVP, up to 9 % where the registers spill (64^3 channel 245 -> 249 us,
+// 56^3 with five species 372 -> 378, 60,000 tetrahedra with nine 398 -> 436); with the second round as a loop around
+// the first, and one copy of the flux, 252, 386 and 433 us.
 template <int DIM, int NS, class G, int FK, bool TAN = false>
 __global__ void __launch_bounds__(128, MinBlocks<NS, G>::tile) k_tile_flux(DevMesh M, Phys P, const double* __restrict__ U,
                                                                      const double* __restrict__ dU, const double* __restrict__ tmp,
